@@ -107,30 +107,9 @@ __host__ __device__ __forceinline__ float tab_sample(const float* col, float nm)
     return a + (b - a) * frac;
 }
 
-// ---- optics (spectral-core/src/optics.rs:8-49) ----------------------------
+// ---- optics (spectral-core/src/optics.rs:8-49; refraction and the Fresnel
+// reflectance are in scatter() below) ----
 __device__ __forceinline__ f3 reflect3(f3 d, f3 n) { return sub(d, mul(n, 2.0f * dot(d, n))); }
-__device__ __forceinline__ bool refract3(f3 d, f3 n, float n1, float n2, f3& out) {
-    float eta = n1 / n2;
-    f3 nn = n;
-    float cos_i = -dot(d, n);
-    if (cos_i < 0.0f) { nn = neg(n); cos_i = -cos_i; }
-    float k = 1.0f - eta * eta * (1.0f - cos_i * cos_i);
-    if (k < 0.0f) return false;
-    float cos_t = sqrtf(k);
-    out = normalize(add(mul(d, eta), mul(nn, eta * cos_i - cos_t)));
-    return true;
-}
-__device__ __forceinline__ float fresnel(float cos_i, float n1, float n2) {
-    cos_i = fminf(fmaxf(cos_i, 0.0f), 1.0f);
-    float e = n1 / n2;
-    float sin_t2 = e * e * (1.0f - cos_i * cos_i);
-    if (sin_t2 >= 1.0f) return 1.0f;
-    float cos_t = sqrtf(1.0f - sin_t2);
-    float rs = (n1 * cos_i - n2 * cos_t) / (n1 * cos_i + n2 * cos_t);
-    float rp = (n1 * cos_t - n2 * cos_i) / (n1 * cos_t + n2 * cos_i);
-    return 0.5f * (rs * rs + rp * rp);
-}
-
 // ---- scene in shared memory ------------------------------------------------
 struct SceneView {
     const sc_primitive* prims;
@@ -140,6 +119,14 @@ struct SceneView {
 };
 struct Hit { float t; f3 point, normal; bool front_face; };
 
+// Whether num / a (a > 0) is certainly below tmin, decided without the division:
+// num below 0.9 tmin a puts the rounded quotient below tmin whatever the
+// rounding (tmin is far from the subnormals).  Comparisons with NaN are false, so
+// such a ray divides as before.
+__device__ __forceinline__ bool below_tmin(float num, float a, float tmin) { return num < 0.9f * tmin * a; }
+
+// Most rays that meet a sphere again start on it: the root they start from is
+// rejected without its division, and so are both roots of a ray that leaves.
 __device__ __forceinline__ bool sphere_hit(const sc_primitive& pr, f3 o, f3 d, float tmin, float tmax, Hit& h) {
     f3 c = ld3(pr.center);
     f3 oc = sub(o, c);
@@ -149,8 +136,14 @@ __device__ __forceinline__ bool sphere_hit(const sc_primitive& pr, f3 o, f3 d, f
     float disc = half_b * half_b - a * cc;
     if (disc < 0.0f) return false;
     float sq = sqrtf(disc);
-    float t = (-half_b - sq) / a;
-    if (t < tmin || t > tmax) {
+    float t = 0.0f;
+    bool near_ok = !below_tmin(-half_b - sq, a, tmin);
+    if (near_ok) {
+        t = (-half_b - sq) / a;
+        near_ok = !(t < tmin || t > tmax);
+    }
+    if (!near_ok) {
+        if (below_tmin(-half_b + sq, a, tmin)) return false;
         t = (-half_b + sq) / a;
         if (t < tmin || t > tmax) return false;
     }
@@ -160,9 +153,15 @@ __device__ __forceinline__ bool sphere_hit(const sc_primitive& pr, f3 o, f3 d, f
     h.t = t; h.point = p; h.normal = ff ? outward : neg(outward); h.front_face = ff;
     return true;
 }
+// Slabs of a convex solid.  Only two kinds of planes need their division: those
+// the ray enters through from outside (denom < 0, dist > 0) and those it leaves
+// from inside (denom > 0, dist < 0).  An entry plane with the origin inside has
+// t <= 0 < tmin: it is never the hit, and when it exceeds t_exit the solid is
+// missed either way.  An exit plane with the origin outside has t <= 0: the solid
+// is behind the ray.  (Comparisons are written so that NaN takes the division.)
 __device__ __forceinline__ bool solid_hit(const SceneView& S, const sc_primitive& pr, f3 o, f3 d, float tmin, float tmax, Hit& h) {
     float t_enter = -__int_as_float(0x7f800000), t_exit = __int_as_float(0x7f800000);
-    f3 en = mk(0.f, 0.f, 0.f), ex = mk(0.f, 0.f, 0.f);
+    uint32_t en = 0xFFFFFFFFu, ex = 0xFFFFFFFFu;  // planes of t_enter and t_exit
     const uint32_t end = pr.plane_start + pr.plane_count;
     for (uint32_t i = pr.plane_start; i < end; ++i) {
         const sc_plane& pl = S.planes[i];
@@ -173,16 +172,23 @@ __device__ __forceinline__ bool solid_hit(const SceneView& S, const sc_primitive
             if (dist > 0.0f) return false;
             continue;
         }
-        float t = -dist / denom;
-        if (denom < 0.0f) { if (t > t_enter) { t_enter = t; en = n; } }
-        else { if (t < t_exit) { t_exit = t; ex = n; } }
+        if (denom < 0.0f) {
+            if (dist <= 0.0f) continue;
+            float t = -dist / denom;
+            if (t > t_enter) { t_enter = t; en = i; }
+        } else {
+            if (dist >= 0.0f) return false;
+            float t = -dist / denom;
+            if (t < t_exit) { t_exit = t; ex = i; }
+        }
     }
     if (t_enter > t_exit) return false;
-    float th; f3 hn;
-    if (t_enter > tmin) { th = t_enter; hn = en; }
-    else if (t_exit > tmin) { th = t_exit; hn = ex; }
+    float th; uint32_t hp;
+    if (t_enter > tmin) { th = t_enter; hp = en; }
+    else if (t_exit > tmin) { th = t_exit; hp = ex; }
     else return false;
     if (th > tmax) return false;
+    f3 hn = hp != 0xFFFFFFFFu ? ld3(S.planes[hp].normal) : mk(0.f, 0.f, 0.f);
     bool ff = dot(hn, d) < 0.0f;
     h.t = th; h.point = add(o, mul(d, th)); h.normal = ff ? hn : neg(hn); h.front_face = ff;
     return true;
@@ -215,13 +221,27 @@ __device__ __forceinline__ f3 cosine_hemisphere(f3 n, Rng& r) {
 }
 __device__ __forceinline__ void scatter(const sc_material& m, f3 wo, const Hit& h, float n_hero, Rng& r, f3& dir, float& w) {
     if (m.kind == 0u) { dir = cosine_hemisphere(h.normal, r); w = m.reflectance; return; }
-    float cos_i = fabsf(-dot(wo, h.normal));
-    float n1 = h.front_face ? 1.0f : n_hero, n2 = h.front_face ? n_hero : 1.0f;
-    float R = fresnel(cos_i, n1, n2);
+    // fresnel() and refract3() in one: both form n1 / n2, the squared sine of the
+    // refracted angle and its cosine, in the same operations while cos_i <= 1
+    // (the cosine fresnel() clamps; a rounded dot product can exceed 1)
+    const float cos_i = fabsf(-dot(wo, h.normal));
+    const float n1 = h.front_face ? 1.0f : n_hero, n2 = h.front_face ? n_hero : 1.0f;
+    const float eta = n1 / n2, c = fminf(fmaxf(cos_i, 0.0f), 1.0f);
+    const float sin_t2 = eta * eta * (1.0f - c * c);
     w = 1.0f;
-    if (r.f32() < R) { dir = reflect3(wo, h.normal); return; }
-    f3 t;
-    if (refract3(wo, h.normal, n1, n2, t)) dir = t; else dir = reflect3(wo, h.normal);
+    const float u = r.f32();
+    bool mirror = true;
+    float cos_t = 0.0f;
+    if (!(sin_t2 >= 1.0f)) {
+        cos_t = sqrtf(1.0f - sin_t2);
+        const float rs = (n1 * c - n2 * cos_t) / (n1 * c + n2 * cos_t);
+        const float rp = (n1 * cos_t - n2 * c) / (n1 * cos_t + n2 * c);
+        mirror = u < 0.5f * (rs * rs + rp * rp);
+    }
+    if (mirror) { dir = reflect3(wo, h.normal); return; }
+    if (cos_i > 1.0f) cos_t = sqrtf(1.0f - eta * eta * (1.0f - cos_i * cos_i));
+    // the normal faces the ray (-wo . n = cos_i)
+    dir = normalize(add(mul(wo, eta), mul(h.normal, eta * cos_i - cos_t)));
 }
 
 // ---- Camera::project with precomputed basis (spectral-core/src/camera.rs:50-69)
