@@ -397,9 +397,8 @@ typedef struct {
 } sc_scene_job;
 /* Tuning knobs, 0 = default: photons per work chunk (queue granularity),
  * register bound (minimum CTAs per SM, 4 or 5), warp-aggregated splats, grid,
- * per_photon = 1 to run each photon's haze samples in its own lane instead
- * of the default warp-split transport (segments buffered per warp, samples
- * processed as one converged list), and threads per CTA (128 or 256). */
+ * per_photon (0 or 1: both run the one transport, photons in groups with each
+ * photon's haze samples in its own lane), and threads per CTA (128 or 256). */
 typedef struct { uint32_t chunk_photons, minb, aggregate, grid, per_photon, block; } sc_batch_tuning;
 int sc_batch_create(sc_ctx* ctx, const sc_scene_job* jobs, uint32_t n_jobs,
                     const sc_batch_tuning* tuning, sc_batch** out);
@@ -414,7 +413,7 @@ int sc_batch_update_jobs(sc_batch* b, const sc_scene_job* jobs, uint32_t n_jobs)
  * Asynchronous; afterwards each job's XYZ image is ready and its film drained. */
 int sc_batch_run(sc_batch* b, void* stream);
 /* The same work as plain per-scene launches (trace + drain/reduce per job),
- * with the transport of the batch's tuning (per_photon). */
+ * in launch order. */
 int sc_batch_run_plain(sc_batch* b, void* stream);
 int sc_batch_synchronize(sc_batch* b);
 int sc_batch_read_xyz(sc_batch* b, uint32_t job, float* out);
@@ -444,8 +443,7 @@ typedef struct {
     uint64_t hbm_budget_bytes;  /* arena for films, masks and images of admitted requests */
     uint32_t max_slots;         /* requests on the device at once (0 -> 256) */
     uint32_t chunk_photons;     /* work-chunk size of the batched launch (0 -> 2048) */
-    uint32_t warp_split;        /* 0: one photon per lane (the default, as the batch autotuner picks
-                                   on uneven scenes); 1: the warp-split transport */
+    uint32_t warp_split;        /* 0 or 1: both run the one transport (see sc_batch_tuning.per_photon) */
 } sc_server_config;
 typedef struct {
     sc_scene_job job;           /* scene, film (bins >= 1), photons per frame (n_photons), seed, camera */

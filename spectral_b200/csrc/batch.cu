@@ -32,7 +32,7 @@ __device__ __forceinline__ void flush_mask(uint32_t* mask, uint32_t words, uint3
 }
 
 // FF: built with free-flight sampling (estimator 3) as well; jobs choose per job.
-template <int AGG, int MINB, bool SPLIT, bool FF>
+template <int AGG, int MINB, bool FF>
 __global__ void __launch_bounds__(256, MINB) batch_kernel(const BatchJobDev* __restrict__ jobs,
                                                           const WorkItem* __restrict__ items, uint32_t n_items,
                                                           uint32_t* counter, const float* __restrict__ cmf_g,
@@ -41,8 +41,7 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const BatchJobDev* __r
     float* cmf = reinterpret_cast<float*>(smem);
     WarpSlot* slots = reinterpret_cast<WarpSlot*>(smem + kCmfBytes16);
     uint32_t* masks = reinterpret_cast<uint32_t*>(slots + blockDim.x / 32);
-    using WS = WarpSplitSmem<kBatchWarpSegs>;
-    WS* split = reinterpret_cast<WS*>(masks + (blockDim.x / 32) * mask_words_max);
+    ParkedPhotons<true>* park = reinterpret_cast<ParkedPhotons<true>*>(masks + (blockDim.x / 32) * mask_words_max);
     for (uint32_t i = threadIdx.x; i < 3u * kTableN; i += blockDim.x) cmf[i] = cmf_g[i];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     uint32_t* mask = masks + warp * mask_words_max;
@@ -71,16 +70,9 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const BatchJobDev* __r
         }
         SceneView S;
         S.prims = slot.prims; S.planes = slot.planes; S.mats = slot.mats; S.n_prims = slot.p.n_prims;
-        if (SPLIT) {
-            const uint32_t first = item.begin;
-            trace_warp_range<true, AGG, FF, kBatchWarpSegs>(slot.p, S, cmf, item.count,
-                                                            [first](uint32_t k) { return first + k; },
-                                                            cur_words ? mask : nullptr, split[warp]);
-        } else {
-            const uint32_t first = item.begin;
-            trace_lane_range<true, AGG, FF>(slot.p, S, cmf, lane, item.count, 32u,
-                                            [first](uint32_t k) { return first + k; }, cur_words ? mask : nullptr);
-        }
+        const uint32_t first = item.begin;
+        trace_group_range<true, AGG, FF>(slot.p, S, cmf, item.count, [first](uint32_t k) { return first + k; },
+                                         cur_words ? mask : nullptr, park[warp]);
         __syncwarp();
     }
     if (cur_words) flush_mask(mask, cur_words, cur_flags, lane);
@@ -88,14 +80,10 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const BatchJobDev* __r
 
 using BatchFn = void (*)(const BatchJobDev*, const WorkItem*, uint32_t, uint32_t*, const float*, uint32_t);
 
-template <bool SPLIT>
-BatchFn batch_fn_t(int agg, int minb, bool ff) {
-    if (ff) return batch_kernel<0, 4, SPLIT, true>;  // batches with free-flight jobs: plain atomics, 4 CTAs per SM
-    if (minb >= 5) return agg ? batch_kernel<1, 5, SPLIT, false> : batch_kernel<0, 5, SPLIT, false>;
-    return agg ? batch_kernel<1, 4, SPLIT, false> : batch_kernel<0, 4, SPLIT, false>;
-}
-BatchFn batch_fn(int agg, int minb, int split, bool ff) {
-    return split ? batch_fn_t<true>(agg, minb, ff) : batch_fn_t<false>(agg, minb, ff);
+BatchFn batch_fn(int agg, int minb, bool ff) {
+    if (ff) return batch_kernel<0, 4, true>;  // batches with free-flight jobs: plain atomics, 4 CTAs per SM
+    if (minb >= 5) return agg ? batch_kernel<1, 5, false> : batch_kernel<0, 5, false>;
+    return agg ? batch_kernel<1, 4, false> : batch_kernel<0, 4, false>;
 }
 
 }  // namespace
@@ -103,29 +91,29 @@ BatchFn batch_fn(int agg, int minb, int split, bool ff) {
 static_assert(sizeof(WarpSlot) % 16 == 0, "warp slot must be a multiple of 16 bytes");
 static_assert(sizeof(WarpSlot) == sizeof(BatchSlotImage), "slot image layout");
 
-size_t batch_smem(uint32_t mask_words_max, int split, uint32_t block) {
+size_t batch_smem(uint32_t mask_words_max, uint32_t block) {
     const size_t warps = block / 32u;
     return kCmfBytes16 + warps * sizeof(WarpSlot) + warps * mask_words_max * sizeof(uint32_t) +
-           (split ? warps * sizeof(WarpSplitSmem<kBatchWarpSegs>) : 0);
+           warps * sizeof(ParkedPhotons<true>);
 }
 
-int batch_occupancy(int agg, int minb, int split, uint32_t mask_words_max, uint32_t block, bool ff) {
+int batch_occupancy(int agg, int minb, uint32_t mask_words_max, uint32_t block, bool ff) {
     int n = 0;
-    const void* fn = reinterpret_cast<const void*>(batch_fn(agg, minb, split, ff));
-    const size_t smem = batch_smem(mask_words_max, split, block);
+    const void* fn = reinterpret_cast<const void*>(batch_fn(agg, minb, ff));
+    const size_t smem = batch_smem(mask_words_max, block);
     if (smem > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)block, smem) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 
 cudaError_t launch_batch(const BatchJobDev* jobs, const WorkItem* items, uint32_t n_items, uint32_t* counter,
-                         const float* cmf, uint32_t mask_words_max, int agg, int minb, int split, uint32_t grid,
+                         const float* cmf, uint32_t mask_words_max, int agg, int minb, uint32_t grid,
                          cudaStream_t s, uint32_t block, bool ff) {
     // the shared-memory attribute was raised by batch_occupancy before any capture
-    const size_t smem = batch_smem(mask_words_max, split, block);
+    const size_t smem = batch_smem(mask_words_max, block);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    batch_fn(agg, minb, split, ff)<<<grid, block, smem, s>>>(jobs, items, n_items, counter, cmf, mask_words_max);
+    batch_fn(agg, minb, ff)<<<grid, block, smem, s>>>(jobs, items, n_items, counter, cmf, mask_words_max);
     return cudaGetLastError();
 }
 

@@ -1,8 +1,7 @@
 // extern "C" batch object: many uneven scenes in one persistent, graph-captured
 // launch (batch.cu), the same work as plain per-scene launches for comparison,
 // and an autotuner that picks chunk size (work-queue granularity), threads per
-// CTA, register bound, splat aggregation and transport by timing the batch
-// itself.
+// CTA, register bound and splat aggregation by timing the batch itself.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -188,8 +187,7 @@ struct sc_batch {
         n.per_photon = n.per_photon ? 1 : 0;
         n.block = n.block == 128u ? 128u : 256u;
         ff = any_free_flight();
-        const int occ = batch_occupancy((int)n.aggregate, (int)n.minb, n.per_photon ? 0 : 1, kBatchMaskWords, n.block,
-                                        ff);
+        const int occ = batch_occupancy((int)n.aggregate, (int)n.minb, kBatchMaskWords, n.block, ff);
         grid = n.grid ? n.grid : (uint32_t)(ctx->sms * occ);
         if (n.chunk_photons != tuning.chunk_photons || n_items == 0) {
             int rc = build_items(n.chunk_photons);
@@ -203,8 +201,7 @@ struct sc_batch {
 
     int enqueue_batch(cudaStream_t s) {
         SC_CUDA(launch_batch(d_jobs.p, d_items.p, n_items, counter.p, ctx->cmf.p, kBatchMaskWords,
-                             (int)tuning.aggregate, (int)tuning.minb, tuning.per_photon ? 0 : 1, grid, s,
-                             tuning.block, ff));
+                             (int)tuning.aggregate, (int)tuning.minb, grid, s, tuning.block, ff));
         // the drain rewrites the images: wait for the last asynchronous copy of them
         SC_CUDA(cudaStreamWaitEvent(s, copied, cudaEventWaitExternal));
         SC_CUDA(launch_reduce_many(d_descs.p, (uint32_t)jobs.size(), total_words, true, max_channels, dirty_list.p,
@@ -244,11 +241,10 @@ struct sc_batch {
                 reinterpret_cast<const unsigned char*>(d_jobs.p + j) + offsetof(BatchSlotImage, planes));
             p.mats = reinterpret_cast<const sc_material*>(
                 reinterpret_cast<const unsigned char*>(d_jobs.p + j) + offsetof(BatchSlotImage, mats));
-            // the transport the batch's tuning chose (measured on these scenes, it
-            // beats the single-film default of warp-split transport plus the
-            // wavelength-ordered dispatch for films larger than L2)
+            // launch order: on these scenes' films it beats the single-film
+            // default (the wavelength-ordered dispatch for films larger than L2)
             LaunchShape shape;
-            shape.block = 256; shape.aggregate = 0; shape.minb = 4; shape.split = tuning.per_photon ? 0 : 1;
+            shape.block = 256; shape.aggregate = 0; shape.minb = 4;
             const size_t smem = scene_smem_bytes(p.n_prims, p.n_planes, p.n_mats) +
                                 (geom[j].words <= kMaxSmemMaskWords ? geom[j].words * 4u : 0u);
             shape.grid = (uint32_t)(ctx->sms * photon_occupancy_blocks(shape, true, smem));
@@ -421,11 +417,10 @@ int sc_batch_autotune(sc_batch* b, sc_batch_tuning* chosen) {
     sc_batch_tuning best{};
     float best_ms = 1e30f;
     for (uint32_t block : {256u, 128u})
-    for (uint32_t per_photon : {0u, 1u})
     for (uint32_t chunk : {512u, 2048u, 8192u})
         for (uint32_t minb : {4u, 5u})
             for (uint32_t agg : {0u, 1u}) {
-                sc_batch_tuning t{chunk, minb, agg, 0, per_photon, block};
+                sc_batch_tuning t{chunk, minb, agg, 0, 1u, block};
                 int rc = b->apply_tuning(t);
                 if (rc == SC_OK) rc = b->run(b->stream);  // warm-up (also builds the graph)
                 if (rc != SC_OK) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
@@ -567,8 +562,7 @@ int sc_batch_stats(sc_batch* b, uint64_t out[6]) {
     SC_CUDA(cudaMemcpyAsync(c, d.p, 32, cudaMemcpyDeviceToHost, b->stream));
     // dirty tiles of one pass: trace only, count the set bits, then drain
     SC_CUDA(launch_batch(b->d_jobs.p, b->d_items.p, b->n_items, b->counter.p, b->ctx->cmf.p, kBatchMaskWords,
-                         (int)b->tuning.aggregate, (int)b->tuning.minb, b->tuning.per_photon ? 0 : 1, b->grid,
-                         b->stream, b->tuning.block, b->ff));
+                         (int)b->tuning.aggregate, (int)b->tuning.minb, b->grid, b->stream, b->tuning.block, b->ff));
     std::vector<uint32_t> fl(b->flags.n);
     SC_CUDA(cudaMemcpyAsync(fl.data(), b->flags.p, b->flags.bytes(), cudaMemcpyDeviceToHost, b->stream));
     SC_CUDA(cudaStreamSynchronize(b->stream));

@@ -74,9 +74,8 @@ static size_t mask_smem(uint32_t w, uint32_t h) {
 }
 
 // The launch shape of single-film traces: 256-thread CTAs, 4 per SM, the
-// warp-split transport, the wavelength-ordered dispatch for spectral films
-// larger than L2.  The environment variables SPECTRAL_CUDA_AGGREGATE,
-// SPECTRAL_CUDA_MINB (4 or 5), SPECTRAL_CUDA_SPLIT (0: one photon per lane) and
+// wavelength-ordered dispatch for spectral films larger than L2.  The environment
+// variables SPECTRAL_CUDA_AGGREGATE, SPECTRAL_CUDA_MINB (4 or 5) and
 // SPECTRAL_CUDA_ORDER (0 never, 1 large spectral films, 2 every spectral film)
 // override it for measurements; every setting gives the same film bits.
 static int default_shape(sc_ctx* ctx, bool spectral, int aggregate, size_t smem, LaunchShape& s,
@@ -86,7 +85,6 @@ static int default_shape(sc_ctx* ctx, bool spectral, int aggregate, size_t smem,
     s.minb = 4;
     if (const char* agg = std::getenv("SPECTRAL_CUDA_AGGREGATE")) s.aggregate = std::atoi(agg) ? 1 : 0;
     if (const char* mb = std::getenv("SPECTRAL_CUDA_MINB")) s.minb = std::atoi(mb) >= 5 ? 5 : 4;
-    if (const char* sp = std::getenv("SPECTRAL_CUDA_SPLIT")) s.split = std::atoi(sp) ? 1 : 0;
     if (const char* od = std::getenv("SPECTRAL_CUDA_ORDER")) s.order = std::min(std::max(std::atoi(od), 0), 2);
     s.pool = ctx->pool;
     const int per_sm = estimator == 2u ? beam_occupancy_blocks(s, spectral, smem)

@@ -42,17 +42,15 @@ struct alignas(16) PhotonParams {
 // Fills the hz_* launch constants of `p` (host side, before every launch).
 void set_haze_consts(PhotonParams& p);
 
-// Photon launch: CTAs of 256 threads, `grid` CTAs (grid-stride), warp
-// aggregation on/off, register bound (minimum CTAs per SM: 4 or 5), the
-// warp-split transport (segments buffered per warp, haze samples processed as
-// one converged list) on/off, and the wavelength-ordered dispatch (0 never,
-// 1 for spectral films larger than L2, 2 for every spectral film; its scratch
-// comes from `pool`, and without a pool it is off).
+// Photon launch: CTAs of 256 threads, `grid` CTAs resident on the GPU at once
+// (the unit the photons are divided by), warp aggregation on/off, register
+// bound (minimum CTAs per SM: 4 or 5), and the wavelength-ordered dispatch (0
+// never, 1 for spectral films larger than L2, 2 for every spectral film; its
+// scratch comes from `pool`, and without a pool it is off).
 struct LaunchShape {
     uint32_t block, grid;
     int aggregate;
     int minb;
-    int split = 1;
     int order = 1;
     cudaMemPool_t pool = nullptr;
 };

@@ -21,9 +21,9 @@ namespace sc {
 
 namespace {
 
-// Byte offset of the warp-split buffers: after scene records, CMF table and the
-// dirty mask, rounded up to 16 bytes.
-__host__ __device__ __forceinline__ size_t split_offset(const PhotonParams& p, uint32_t mask_words) {
+// Byte offset of the warps' parked photons: after scene records, CMF table and
+// the dirty mask, rounded up to 16 bytes.
+__host__ __device__ __forceinline__ size_t park_offset(const PhotonParams& p, uint32_t mask_words) {
     const size_t b = p.n_prims * sizeof(sc_primitive) + p.n_planes * sizeof(sc_plane) +
                      p.n_mats * sizeof(sc_material) + 3 * kTableN * sizeof(float) + mask_words * sizeof(uint32_t);
     return (b + 15u) & ~size_t(15);
@@ -33,40 +33,31 @@ __host__ __device__ __forceinline__ size_t split_offset(const PhotonParams& p, u
 // no spills; 5: 48 registers, a few spills, more warps in flight).
 // FF: built with free-flight sampling (estimator 3) as well.  EXACT: haze
 // samples in the CPU crate's operation order (per-photon transport only).
-template <bool SPEC, int AGG, int MINB, bool SPLIT, bool FF, bool EXACT = false>
-__global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words) {
+// chunk: photons of each warp (not EXACT).
+template <bool SPEC, int AGG, int MINB, bool FF, bool EXACT = false>
+__global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words, uint32_t chunk) {
     extern __shared__ __align__(16) unsigned char smem[];
     const float* cmf;
     uint32_t* smask;
     const SceneView S = load_scene(p, smem, &cmf, &smask, mask_words);
-    if (SPLIT) {  // warp-split transport: per-warp segment buffers after the scene
-        // warps take chunks of the launch's photons in grid-stride order (so the
-        // photons in flight stay close in launch order: the wavelength-ordered
-        // dispatch relies on it), and the lanes work through a chunk with refill;
-        // chunks of up to 512 photons, smaller when that leaves warps idle
-        using WS = WarpSplitSmem<kWarpSegs>;
-        WS* ws = reinterpret_cast<WS*>(smem + split_offset(p, mask_words));
-        const uint32_t warp = threadIdx.x >> 5;
-        const uint32_t warps = gridDim.x * (blockDim.x >> 5), gw = blockIdx.x * (blockDim.x >> 5) + warp;
-        const uint32_t per = (uint32_t)(((uint64_t)p.photon_count + warps - 1u) / warps);
-        const uint32_t chunk = min(512u, max(32u, (per + 31u) & ~31u));
-        for (uint64_t base = (uint64_t)gw * chunk; base < p.photon_count; base += (uint64_t)warps * chunk) {
-            const uint32_t b0 = (uint32_t)base;
-            const uint32_t cnt = min(chunk, p.photon_count - b0);
-            trace_warp_range<SPEC, AGG, FF, kWarpSegs>(
-                p, S, cmf, cnt, [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); },
-                smask, ws[warp]);
-        }
-    } else if (EXACT) {
+    if (EXACT) {
         const uint32_t stride = gridDim.x * blockDim.x;
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.photon_count; i += stride)
             trace_photon<SPEC, AGG, false, false, FF, true>(p, S, cmf, p.photon_base + (p.order ? p.order[i] : i),
                                                              smask);
     } else {
-        trace_lane_range<SPEC, AGG, FF>(p, S, cmf, blockIdx.x * blockDim.x + threadIdx.x, p.photon_count,
-                                        gridDim.x * blockDim.x,
-                                        [&](uint32_t i) { return p.photon_base + (p.order ? p.order[i] : i); },
-                                        smask);
+        // one chunk of the launch's photons per warp; CTAs start in launch order, so
+        // the photons in flight stay close in it (the wavelength-ordered dispatch
+        // relies on that)
+        const uint32_t warp = threadIdx.x >> 5;
+        const uint64_t base = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + warp) * chunk;
+        if (base < p.photon_count) {
+            const uint32_t b0 = (uint32_t)base;
+            trace_group_range<SPEC, AGG, FF>(
+                p, S, cmf, min(chunk, p.photon_count - b0),
+                [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); }, smask,
+                reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp]);
+        }
     }
     if (smask) {  // publish this CTA's dirty tiles
         __syncthreads();
@@ -275,32 +266,27 @@ size_t scene_smem_bytes(uint32_t n_prims, uint32_t n_planes, uint32_t n_mats) {
            3 * kTableN * sizeof(float);
 }
 
-using PhotonKernelFn = void (*)(const PhotonParams, uint32_t);
+using PhotonKernelFn = void (*)(const PhotonParams, uint32_t, uint32_t);
 
-template <bool SPLIT>
-static PhotonKernelFn photon_fn_t(bool spec, int agg, int minb, bool ff, bool exact) {
+static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool ff, bool exact = false) {
     // haze samples in the reference's operation order: per-photon transport,
     // plain atomics, 4 CTAs per SM
-    if (exact && !SPLIT) {
-        if (ff) return spec ? photon_kernel<true, 0, 4, false, true, true> : photon_kernel<false, 0, 4, false, true, true>;
-        return spec ? photon_kernel<true, 0, 4, false, false, true> : photon_kernel<false, 0, 4, false, false, true>;
+    if (exact) {
+        if (ff) return spec ? photon_kernel<true, 0, 4, true, true> : photon_kernel<false, 0, 4, true, true>;
+        return spec ? photon_kernel<true, 0, 4, false, true> : photon_kernel<false, 0, 4, false, true>;
     }
     // free-flight launches: plain atomics, 4 CTAs per SM
-    if (ff) return spec ? photon_kernel<true, 0, 4, SPLIT, true> : photon_kernel<false, 0, 4, SPLIT, true>;
-    if (minb >= 5) {
-        if (spec) return agg ? photon_kernel<true, 1, 5, SPLIT, false> : photon_kernel<true, 0, 5, SPLIT, false>;
-        return agg ? photon_kernel<false, 1, 5, SPLIT, false> : photon_kernel<false, 0, 5, SPLIT, false>;
+    if (ff) return spec ? photon_kernel<true, 0, 4, true> : photon_kernel<false, 0, 4, true>;
+    if (s.minb >= 5) {
+        if (spec) return s.aggregate ? photon_kernel<true, 1, 5, false> : photon_kernel<true, 0, 5, false>;
+        return s.aggregate ? photon_kernel<false, 1, 5, false> : photon_kernel<false, 0, 5, false>;
     }
-    if (spec) return agg ? photon_kernel<true, 1, 4, SPLIT, false> : photon_kernel<true, 0, 4, SPLIT, false>;
-    return agg ? photon_kernel<false, 1, 4, SPLIT, false> : photon_kernel<false, 0, 4, SPLIT, false>;
+    if (spec) return s.aggregate ? photon_kernel<true, 1, 4, false> : photon_kernel<true, 0, 4, false>;
+    return s.aggregate ? photon_kernel<false, 1, 4, false> : photon_kernel<false, 0, 4, false>;
 }
-static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool ff, bool exact = false) {
-    return s.split && !exact ? photon_fn_t<true>(spec, s.aggregate, s.minb, ff, false)
-                             : photon_fn_t<false>(spec, s.aggregate, s.minb, ff, exact);
-}
-// Shared memory beyond scene + mask: one segment buffer per warp (8 warps).
-static size_t split_bytes(const LaunchShape& s) {
-    return s.split ? 16 + 8 * sizeof(WarpSplitSmem<kWarpSegs>) : 0;
+// Shared memory beyond scene + mask: the parked photons of 8 warps.
+static size_t park_bytes(bool spec) {
+    return 16 + 8 * (spec ? sizeof(ParkedPhotons<true>) : sizeof(ParkedPhotons<false>));
 }
 
 void set_haze_consts(PhotonParams& p) {
@@ -339,7 +325,7 @@ int occupancy_blocks(const void* fn, int block, size_t smem) {
 
 int photon_occupancy_blocks(const LaunchShape& shape, bool spectral, size_t smem) {
     return occupancy_blocks(reinterpret_cast<const void*>(photon_fn(shape, spectral, false)), (int)shape.block,
-                            smem + split_bytes(shape));
+                            smem + park_bytes(spectral));
 }
 
 uint32_t photon_mask_words(const PhotonParams& p) {
@@ -412,15 +398,27 @@ static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& 
     set_haze_consts(p);
     const bool exact = p.haze_exact != 0u;
     const uint32_t mw = photon_mask_words(p);
-    const size_t smem = shape.split && !exact
-                            ? split_offset(p, mw) + 8 * sizeof(WarpSplitSmem<kWarpSegs>)
-                            : scene_smem_bytes(p.n_prims, p.n_planes, p.n_mats) + mw * sizeof(uint32_t);
     const bool spec = p.channels != 3u || p.bins != 0u;
-    const uint32_t need = (p.photon_count + 255u) / 256u;
-    const uint32_t grid = need < shape.grid ? need : shape.grid;
+    const size_t smem = park_offset(p, mw) + park_bytes(spec);
     const PhotonKernelFn fn = photon_fn(shape, spec, free_flight(p), exact);
     if (smem > 48 * 1024) occupancy_blocks(reinterpret_cast<const void*>(fn), 256, smem);  // raises its limit once
-    fn<<<grid, 256, smem, s>>>(p, mw);
+    uint32_t chunk = 0, grid;
+    if (exact) {
+        const uint32_t need = (p.photon_count - 1u) / 256u + 1u;
+        grid = need < shape.grid ? need : shape.grid;
+    } else {
+        // About two chunks for each warp the GPU holds, 64 to 256 photons: the
+        // hardware starts the next CTA where one has ended.  One CTA per resident
+        // slot with its share of the photons ended unevenly (rainbow, 2^26 photons:
+        // 8.3 ms against 6.75; SMs idle 18 % of it); longer chunks do so again (512:
+        // 6.79 ms, 2048: 6.98), shorter ones pay for each warp's last photons and
+        // each CTA's setup (2^26 photons in chunks of 64: 7.35 ms; 2^20: 128 219 us,
+        // 64 222, 256 255; 2^16: 64 139 us, 32 146, 256 174).
+        const uint64_t per = p.photon_count / (shape.grid * 16ull);
+        chunk = (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
+        grid = (uint32_t)((p.photon_count - 1u) / (8ull * chunk) + 1u);
+    }
+    fn<<<grid, 256, smem, s>>>(p, mw, chunk);
     return cudaGetLastError();
 }
 
