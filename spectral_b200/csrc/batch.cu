@@ -101,7 +101,7 @@ int batch_occupancy(int agg, int minb, uint32_t mask_words_max, uint32_t block, 
     int n = 0;
     const void* fn = reinterpret_cast<const void*>(batch_fn(agg, minb, ff));
     const size_t smem = batch_smem(mask_words_max, block);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_max_smem(fn);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)block, smem) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }

@@ -626,8 +626,7 @@ cudaError_t launch_beam_count(const PhotonParams& p, unsigned long long* out, ui
     const uint32_t need = (p.photon_count + 255u) / 256u;
     const size_t smem = beam_smem(p, 0);
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute(reinterpret_cast<const void*>(beam_count_kernel),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_max_smem(reinterpret_cast<const void*>(beam_count_kernel));
     beam_count_kernel<<<need < grid ? need : grid, 256, smem, s>>>(p, out);
     return cudaGetLastError();
 }

@@ -397,7 +397,7 @@ static uint32_t reduce_grid(const void* fn, int which, size_t smem) {
     if (it != cache.end()) return it->second;
     int sms = 148, per_sm = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_max_smem(fn);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kReduceThreads, smem);
     const uint32_t grid = (uint32_t)sms * (uint32_t)(per_sm > 0 ? per_sm : 1);
     cache.emplace(key, grid);

@@ -11,9 +11,12 @@
 // Splats land in a 64-bit fixed-point film with red.global.add.u64; the film is
 // tile-major (8x8 pixel tiles) and every touched tile raises a dirty flag so the
 // drain/reduce pass reads only tiles that received light.
+#include <cmath>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
+#include <utility>
 
 #include "photon_trace.cuh"
 
@@ -33,9 +36,11 @@ __host__ __device__ __forceinline__ size_t park_offset(const PhotonParams& p, ui
 // no spills; 5: 48 registers, a few spills, more warps in flight).
 // FF: built with free-flight sampling (estimator 3) as well.  EXACT: haze
 // samples in the CPU crate's operation order (per-photon transport only).
-// chunk: photons of each warp (not EXACT).
-template <bool SPEC, int AGG, int MINB, bool FF, bool EXACT = false>
-__global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words, uint32_t chunk) {
+// CACHE: built with the shared-memory cell cache.  chunk: photons of each warp
+// (not EXACT).  cached: use the cache (CACHE only).
+template <bool SPEC, int AGG, int MINB, bool FF, bool EXACT = false, bool CACHE = false>
+__global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words, uint32_t chunk,
+                                                           uint32_t cached) {
     extern __shared__ __align__(16) unsigned char smem[];
     const float* cmf;
     uint32_t* smask;
@@ -46,6 +51,13 @@ __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p,
             trace_photon<SPEC, AGG, false, false, FF, true>(p, S, cmf, p.photon_base + (p.order ? p.order[i] : i),
                                                              smask);
     } else {
+        CellCacheOf<SPEC>* cache = nullptr;
+        if (CACHE && cached) {
+            cache = reinterpret_cast<CellCacheOf<SPEC>*>(smem + park_offset(p, mask_words) +
+                                                         8 * sizeof(ParkedPhotons<SPEC>));
+            cache->clear();
+            __syncthreads();
+        }
         // one chunk of the launch's photons per warp; CTAs start in launch order, so
         // the photons in flight stay close in it (the wavelength-ordered dispatch
         // relies on that)
@@ -56,7 +68,11 @@ __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p,
             trace_group_range<SPEC, AGG, FF>(
                 p, S, cmf, min(chunk, p.photon_count - b0),
                 [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); }, smask,
-                reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp]);
+                reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp], cache);
+        }
+        if (CACHE && cached) {
+            __syncthreads();
+            cache->flush(p.film);
         }
     }
     if (smask) {  // publish this CTA's dirty tiles
@@ -266,9 +282,10 @@ size_t scene_smem_bytes(uint32_t n_prims, uint32_t n_planes, uint32_t n_mats) {
            3 * kTableN * sizeof(float);
 }
 
-using PhotonKernelFn = void (*)(const PhotonParams, uint32_t, uint32_t);
+using PhotonKernelFn = void (*)(const PhotonParams, uint32_t, uint32_t, uint32_t);
 
-static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool ff, bool exact = false) {
+// `few`: film of few cells per pixel (the kernels built with the cell cache).
+static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool few, bool ff, bool exact = false) {
     // haze samples in the reference's operation order: per-photon transport,
     // plain atomics, 4 CTAs per SM
     if (exact) {
@@ -276,17 +293,24 @@ static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool ff, bool e
         return spec ? photon_kernel<true, 0, 4, false, true> : photon_kernel<false, 0, 4, false, true>;
     }
     // free-flight launches: plain atomics, 4 CTAs per SM
-    if (ff) return spec ? photon_kernel<true, 0, 4, true> : photon_kernel<false, 0, 4, true>;
-    if (s.minb >= 5) {
-        if (spec) return s.aggregate ? photon_kernel<true, 1, 5, false> : photon_kernel<true, 0, 5, false>;
-        return s.aggregate ? photon_kernel<false, 1, 5, false> : photon_kernel<false, 0, 5, false>;
+    if (ff) {
+        if (!spec) return photon_kernel<false, 0, 4, true, false, true>;
+        return few ? photon_kernel<true, 0, 4, true, false, true> : photon_kernel<true, 0, 4, true>;
     }
-    if (spec) return s.aggregate ? photon_kernel<true, 1, 4, false> : photon_kernel<true, 0, 4, false>;
-    return s.aggregate ? photon_kernel<false, 1, 4, false> : photon_kernel<false, 0, 4, false>;
+    if (s.aggregate) {
+        if (s.minb >= 5) return spec ? photon_kernel<true, 1, 5, false> : photon_kernel<false, 1, 5, false>;
+        return spec ? photon_kernel<true, 1, 4, false> : photon_kernel<false, 1, 4, false>;
+    }
+    if (few) {  // the cache's shared memory holds 3 CTAs per SM
+        return spec ? photon_kernel<true, 0, 4, false, false, true> : photon_kernel<false, 0, 4, false, false, true>;
+    }
+    return s.minb >= 5 ? photon_kernel<true, 0, 5, false> : photon_kernel<true, 0, 4, false>;
 }
-// Shared memory beyond scene + mask: the parked photons of 8 warps.
-static size_t park_bytes(bool spec) {
-    return 16 + 8 * (spec ? sizeof(ParkedPhotons<true>) : sizeof(ParkedPhotons<false>));
+static bool few_cells(bool spec, uint32_t channels) { return !spec || channels <= kCacheBins; }
+// Shared memory beyond scene + mask: the parked photons of 8 warps, the cache.
+static size_t park_bytes(bool spec, bool cached) {
+    return 16 + (spec ? 8 * sizeof(ParkedPhotons<true>) + (cached ? sizeof(CellCacheOf<true>) : 0)
+                      : 8 * sizeof(ParkedPhotons<false>) + (cached ? sizeof(CellCacheOf<false>) : 0));
 }
 
 void set_haze_consts(PhotonParams& p) {
@@ -306,17 +330,36 @@ void set_haze_consts(PhotonParams& p) {
     p.hz_m2g = (float)(-2.0 * g);
 }
 
+void allow_max_smem(const void* fn) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({dev, fn})) return;
+    cudaFuncAttributes at;
+    int optin = 0;
+    if (cudaFuncGetAttributes(&at, fn) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)at.sharedSizeBytes) !=
+            cudaSuccess) {
+        cudaGetLastError();  // a launch that needs more then reports it
+        return;
+    }
+    done.insert({dev, fn});
+}
+
 int occupancy_blocks(const void* fn, int block, size_t smem) {
     static std::mutex mu;
     static std::map<std::tuple<int, const void*, int, size_t>, int> cache;
     int dev = 0;
     cudaGetDevice(&dev);
+    if (smem > 48 * 1024) allow_max_smem(fn);
     std::lock_guard<std::mutex> lk(mu);
     const auto key = std::make_tuple(dev, fn, block, smem);
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
     int n = 0;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, block, smem) != cudaSuccess) return 1;
     n = n > 0 ? n : 1;
     cache.emplace(key, n);
@@ -324,8 +367,8 @@ int occupancy_blocks(const void* fn, int block, size_t smem) {
 }
 
 int photon_occupancy_blocks(const LaunchShape& shape, bool spectral, size_t smem) {
-    return occupancy_blocks(reinterpret_cast<const void*>(photon_fn(shape, spectral, false)), (int)shape.block,
-                            smem + park_bytes(spectral));
+    return occupancy_blocks(reinterpret_cast<const void*>(photon_fn(shape, spectral, !spectral, false)),
+                            (int)shape.block, smem + park_bytes(spectral, false));
 }
 
 uint32_t photon_mask_words(const PhotonParams& p) {
@@ -393,32 +436,59 @@ cudaError_t launch_photons(const PhotonParams& p, const LaunchShape& shape, cuda
     return e != cudaSuccess ? e : f;
 }
 
+// Whether the cell cache pays: the launch is not small (2^14 photons take as long
+// with it as without: clearing and flushing it is 3 us), and the 32 * chunk
+// first-segment samples of a CTA share cells.  These lie along the beam: the
+// frame's height times the beam's width in pixels, seen from the camera at the
+// beam's start.  Measured at 640x360 (width 2 to 3 pixels): XYZ, 2^16 photons
+// 62 -> 39 us (dsotm), 97 -> 56 (prism), 2^20 641 -> 250, 1017 -> 449; 8 bins, 2^20
+// 212 -> 200, 367 -> 236 (4 samples a cell at XYZ 2^20).  The rainbow's beam (205
+// pixels): XYZ 2^20 325 -> 277 us (0.055 samples a cell), 2^18 103 -> 92 and 2 bins
+// 2^20 162 -> 152 (0.028), but 4 bins 2^20 108 -> 146 and XYZ 2^15 24 -> 29 (0.014):
+// the line lies at 0.02.  A z-buffer takes samples away: 0.055 then lose (148 ->
+// 201), 4 still win (prism 995 -> 464).
+static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk) {
+    if (p.photon_count < (1u << 15)) return false;
+    const f3 c = sub(add(p.corner, mul(add(p.bu, p.bv), 0.5f)), p.proj.o);
+    const float depth = -dot(c, p.proj.w) / length(p.proj.w);
+    const f3 across = cross(p.bdir, p.proj.w);  // on screen, square to the beam
+    const float l = length(across);
+    float width = length(p.bu) + length(p.bv);
+    if (l > 1e-3f * length(p.bdir) * length(p.proj.w)) width = (fabsf(dot(p.bu, across)) + fabsf(dot(p.bv, across))) / l;
+    if (!(depth > 0.0f)) return false;
+    const float pixels = (1.0f + width / depth * (float)p.height / p.proj.vh) * (float)p.height;
+    return 32.0f * (float)chunk >= (p.zbuf ? 0.4f : 0.02f) * pixels * (float)cells_per_pixel;
+}
+
 static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& shape, cudaStream_t s) {
     PhotonParams p = p0;
     set_haze_consts(p);
     const bool exact = p.haze_exact != 0u;
     const uint32_t mw = photon_mask_words(p);
-    const bool spec = p.channels != 3u || p.bins != 0u;
-    const size_t smem = park_offset(p, mw) + park_bytes(spec);
-    const PhotonKernelFn fn = photon_fn(shape, spec, free_flight(p), exact);
-    if (smem > 48 * 1024) occupancy_blocks(reinterpret_cast<const void*>(fn), 256, smem);  // raises its limit once
+    const bool spec = p.channels != 3u || p.bins != 0u, few = few_cells(spec, p.channels);
     uint32_t chunk = 0, grid;
     if (exact) {
         const uint32_t need = (p.photon_count - 1u) / 256u + 1u;
         grid = need < shape.grid ? need : shape.grid;
     } else {
-        // About two chunks for each warp the GPU holds, 64 to 256 photons: the
-        // hardware starts the next CTA where one has ended.  One CTA per resident
-        // slot with its share of the photons ended unevenly (rainbow, 2^26 photons:
-        // 8.3 ms against 6.75; SMs idle 18 % of it); longer chunks do so again (512:
-        // 6.79 ms, 2048: 6.98), shorter ones pay for each warp's last photons and
-        // each CTA's setup (2^26 photons in chunks of 64: 7.35 ms; 2^20: 128 219 us,
-        // 64 222, 256 255; 2^16: 64 139 us, 32 146, 256 174).
-        const uint64_t per = p.photon_count / (shape.grid * 16ull);
-        chunk = (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
+        // 32 photons for each warp while the GPU holds all of them; then about two
+        // chunks for each warp that it holds, 64 to 256 photons: the hardware starts
+        // the next CTA where one has ended.  One CTA per resident slot with its share
+        // of the photons ended unevenly (rainbow, 2^26 photons: 8.3 ms against 6.75,
+        // SMs idle 18 % of it); longer chunks do so again (512: 6.79 ms, 2048: 6.98),
+        // shorter ones pay for each warp's last photons and each CTA's setup (2^26
+        // photons in chunks of 64: 7.35 ms; 2^20 photons, 32 bins: 32 210 us, 64 195,
+        // 128 205, 256 230; 2^16: 32 29 us, 64 33, 128 52).
+        const uint64_t held = shape.grid * 8ull, per = p.photon_count / (2ull * held);
+        chunk = p.photon_count <= 32ull * held ? 32u
+                                               : (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
         grid = (uint32_t)((p.photon_count - 1u) / (8ull * chunk) + 1u);
     }
-    fn<<<grid, 256, smem, s>>>(p, mw, chunk);
+    const bool cached = !exact && few && shape.aggregate == 0 && cache_pays(p, spec ? p.channels : 1u, chunk);
+    const size_t smem = park_offset(p, mw) + (exact ? 0 : park_bytes(spec, cached));
+    const PhotonKernelFn fn = photon_fn(shape, spec, few, free_flight(p), exact);
+    if (smem > 48 * 1024) allow_max_smem(reinterpret_cast<const void*>(fn));
+    fn<<<grid, 256, smem, s>>>(p, mw, chunk, cached ? 1u : 0u);
     return cudaGetLastError();
 }
 

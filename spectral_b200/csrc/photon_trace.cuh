@@ -73,13 +73,78 @@ __device__ __forceinline__ FilmView film_view(const PhotonParams& p, uint32_t bi
     return v;
 }
 
+// Shared-memory sums of the film cells a CTA deposits to most often, for films
+// with few cells per pixel: the photons of a narrow beam meet in a few hundred
+// pixels, and every photon of the launch adds to the same cells of each.  L2 adds
+// to one 128-byte line a few times slower than to several (XYZ films took 3 to 5
+// times as long as 32-bin films of the same photons).  A cell (the three of an XYZ
+// pixel, the one of a spectral film's pixel and bin) takes the slot its hash names
+// if that is free; others go straight to the film.  Sums are two 32-bit words per
+// value (12 low bits, and the rest), so that values below 2^23 stay exact over
+// 2^20 deposits, more than a CTA makes (8 warps x 256 photons x 64 bounces x 4).
+// V: values per cell.
+template <int V>
+struct CellCache {
+    static constexpr uint32_t kLog2 = V == 3 ? 11u : 12u, kSlots = 1u << kLog2;
+    static constexpr uint32_t kFree = 0xFFFFFFFFu;
+    uint32_t key[kSlots];         // pixel (tile-major) x cells of a pixel + bin, or free
+    uint32_t sum[2 * V][kSlots];  // low and high words of the values
+    __device__ __forceinline__ void clear() {
+        for (uint32_t i = threadIdx.x; i < kSlots; i += blockDim.x) {
+            key[i] = kFree;
+#pragma unroll
+            for (int k = 0; k < 2 * V; ++k) sum[k][i] = 0u;
+        }
+    }
+    // Adds the sums to the film; key k is V-tuple k of its cells.
+    __device__ __forceinline__ void flush(unsigned long long* film) const {
+        for (uint32_t i = threadIdx.x; i < kSlots; i += blockDim.x) {
+            if (key[i] == kFree) continue;
+            unsigned long long* cell = film + (size_t)key[i] * V;
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                red_u64(cell + k, (unsigned long long)sum[2 * k][i] + ((unsigned long long)sum[2 * k + 1][i] << 12));
+        }
+    }
+    // Whether the values went into the cache.
+    __device__ __forceinline__ bool add(uint32_t k, const unsigned long long (&v)[V]) {
+        unsigned long long any = 0;
+#pragma unroll
+        for (int c = 0; c < V; ++c) any |= v[c];
+        if (any >> 23) return false;
+        const uint32_t slot = (k * 0x9E3779B1u) >> (32u - kLog2);
+        uint32_t t = key[slot];
+        if (t == kFree) t = atomicCAS(&key[slot], kFree, k);
+        if (t != k && t != kFree) return false;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            atomicAdd(&sum[2 * c][slot], (uint32_t)v[c] & 0xFFFu);
+            atomicAdd(&sum[2 * c + 1][slot], (uint32_t)v[c] >> 12);
+        }
+        return true;
+    }
+};
+// Spectral films of up to this many bins may go through the cache (2^20 photons
+// of the narrow prism beam: 1 bin 1053 -> 239 us, 4 bins 387 -> 223, 8 bins
+// 367 -> 236; 16 bins take 218 without it, 32 bins 200).
+constexpr uint32_t kCacheBins = 8;
+// No cache (a null pointer of it): films of many bins, and small launches.
+template <bool SPEC> using CellCacheOf = CellCache<SPEC ? 1 : 3>;
+
+template <bool SPEC>
+__device__ __forceinline__ bool cache_take(CellCacheOf<SPEC>& cache, const PhotonParams& p, uint32_t pixel, uint32_t bin,
+                                           unsigned long long v0, unsigned long long v1, unsigned long long v2) {
+    if constexpr (SPEC) return cache.add(pixel * p.channels + bin, {v0});
+    else return cache.add(pixel, {v0, v1, v2});
+}
+
 // Deposit one haze sample.  AGG=1 merges lanes of the warp that hit the same
 // film cell before issuing the atomic.
 // `scale`: the film's 2^k, or 1 when `contrib` carries it already.
 template <bool SPEC, int AGG>
 __device__ __forceinline__ void deposit(const PhotonParams& p, const FilmView& fv, uint32_t* smask, bool ok,
                                         uint32_t px, uint32_t py, float contrib, float cx, float cy, float cz,
-                                        float scale) {
+                                        float scale, CellCacheOf<SPEC>* cache = nullptr, uint32_t bin = 0) {
     unsigned long long* cell = nullptr;
     uint32_t tile = 0, pixel = 0;
     unsigned long long v0 = 0, v1 = 0, v2 = 0;
@@ -98,6 +163,7 @@ __device__ __forceinline__ void deposit(const PhotonParams& p, const FilmView& f
     if (AGG == 0) {
         if (!ok) return;
         mark_tile(p, smask, tile);
+        if (cache && cache_take<SPEC>(*cache, p, pixel, bin, v0, v1, v2)) return;
         red_u64(cell, v0);
         if (!SPEC) { red_u64(cell + 1, v1); red_u64(cell + 2, v2); }
         return;
@@ -404,12 +470,13 @@ __device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneV
 }
 
 // The four haze samples of a segment into the film.  With plain atomics and the
-// uniform point estimator (no z-buffer), all four are worked out before the
-// first deposit, without a branch, so that their chains of approximations
-// overlap: batch pass 22.3 -> 20.5 ms against sample by sample.  G: g != 0.
+// uniform point estimator, all four are worked out before the first deposit,
+// without a branch, so that their chains of approximations overlap: batch pass
+// 22.3 -> 20.5 ms against sample by sample.  (Not with a z-buffer: a sample that
+// is occluded ends there.)  G: g != 0.
 template <bool SPEC, bool G>
 __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& h, Rng& r, float cx, float cy, float cz,
-                                          uint32_t bin, uint32_t* smask) {
+                                          uint32_t bin, uint32_t* smask, CellCacheOf<SPEC>* cache) {
     const HazeView v = haze_view(p);
     const FilmView fv = film_view(p, SPEC ? bin : 0u);
     uint32_t pixel[4];
@@ -442,11 +509,16 @@ __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& 
             unsigned long long* cell = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(fv.cell0) +
                                                                              (size_t)pixel[k] * fv.stride);
             if (SPEC) {
-                red_u64(cell, to_fixed(weight[k], 1.0f));
+                const unsigned long long x = to_fixed(weight[k], 1.0f);
+                if (!cache || !cache_take<SPEC>(*cache, p, pixel[k], bin, x, 0ull, 0ull)) red_u64(cell, x);
             } else {
-                red_u64(cell, to_fixed(cx * weight[k], 1.0f));
-                red_u64(cell + 1, to_fixed(cy * weight[k], 1.0f));
-                red_u64(cell + 2, to_fixed(cz * weight[k], 1.0f));
+                const unsigned long long x = to_fixed(cx * weight[k], 1.0f), y = to_fixed(cy * weight[k], 1.0f),
+                                         z = to_fixed(cz * weight[k], 1.0f);
+                if (!cache || !cache_take<SPEC>(*cache, p, pixel[k], 0u, x, y, z)) {
+                    red_u64(cell, x);
+                    red_u64(cell + 1, y);
+                    red_u64(cell + 2, z);
+                }
             }
         }
     }
@@ -472,7 +544,8 @@ constexpr int kGroupLive = 24;
 // bit-identical to it.
 template <bool SPEC, int AGG, bool FFOK, class Id>
 __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const SceneView& S, const float* cmf,
-                                                  uint32_t count, Id id, uint32_t* smask, ParkedPhotons<SPEC>& park) {
+                                                  uint32_t count, Id id, uint32_t* smask, ParkedPhotons<SPEC>& park,
+                                                  CellCacheOf<SPEC>* cache = nullptr) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     const bool ff = FFOK && free_flight(p);
@@ -547,8 +620,8 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
             const float seg = any ? h.t : p.max_dist;
             const HazeSeg hz = ff ? haze_setup<true>(p, o, d, seg, power) : haze_setup<false>(p, o, d, seg, power);
             if (AGG == 0 && !ff && !p.zbuf && p.estimator != 1u) {
-                if (p.g == 0.0f) haze_four<SPEC, false>(p, hz, r, cx, cy, cz, bin, smask);
-                else haze_four<SPEC, true>(p, hz, r, cx, cy, cz, bin, smask);
+                if (p.g == 0.0f) haze_four<SPEC, false>(p, hz, r, cx, cy, cz, bin, smask, cache);
+                else haze_four<SPEC, true>(p, hz, r, cx, cy, cz, bin, smask, cache);
             } else {
                 const HazeView hv = haze_view(p);
                 const FilmView fv = film_view(p, SPEC ? bin : 0u);
@@ -559,7 +632,7 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
                     float contrib;
                     const bool ok = ff ? haze_fast<true>(p, hv, hz, draw24, px, py, contrib)
                                        : haze_fast<false>(p, hv, hz, draw24, px, py, contrib);
-                    deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f);
+                    deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f, cache, bin);
                 }
             }
             ++bounce;
