@@ -1,6 +1,9 @@
 // Batched uneven workload: device structures shared by batch.cu (kernel) and
 // batch_api.cu (host object).
 #pragma once
+#include <algorithm>
+#include <vector>
+
 #include "photon_trace.cuh"
 
 namespace sc {
@@ -26,6 +29,30 @@ struct alignas(16) BatchJobDev {
 };
 
 struct WorkItem { uint32_t job, begin, count; };
+
+// Appends the work items of photons [begin, begin + count) of job `job` to `out`.
+// `left`: photons of the whole launch not yet cut, this job's included; `warps`:
+// warps that share the launch.  An item is at most `chunk` photons and at most an
+// even share of what is left (half of one while shares are large), but not below
+// kMinChunk: large items keep a warp on one film, small ones at the end let the
+// warps finish together, and a launch of few photons is spread over all warps.
+// Fixed items left most warps idle where there were fewer items than warps.
+// Measured against fixed items: 256 scenes, chunk 8192 21.1 -> 19.3 ms; 16 scenes
+// of up to 2^20 photons 3.5 -> 0.66 ms; 40 served requests (chunk 2048) 163 -> 122
+// ms.  Half shares throughout: 19.3, 0.77, 130; whole ones: 19.6, 0.66, 122.
+constexpr uint32_t kMinChunk = 64;
+inline void cut_items(std::vector<WorkItem>& out, uint32_t job, uint32_t begin, uint32_t count, uint32_t chunk,
+                      uint64_t& left, uint32_t warps) {
+    while (count) {
+        uint64_t share = left / std::max(warps, 1u) + 31u;
+        if (share >= 1024u) share /= 2u;
+        const uint32_t n = std::min({count, chunk, std::max(kMinChunk, (uint32_t)std::min<uint64_t>(share, chunk) & ~31u)});
+        out.push_back(WorkItem{job, begin, n});
+        begin += n;
+        count -= n;
+        left -= n;
+    }
+}
 
 // `block`: threads per CTA, 128 or 256 (one shared-memory job slot per warp).
 // `ff`: some job uses free-flight sampling (the kernel built with it).

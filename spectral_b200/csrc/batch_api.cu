@@ -82,6 +82,7 @@ struct sc_batch {
         h_stage = nullptr;
         staged = nullptr;
     }
+    uint32_t items_warps = 0;  // warps the items are cut for
     uint32_t n_items = 0, total_tiles = 0, total_words = 0, max_channels = 0;
     uint64_t total_photons = 0;
     sc_batch_tuning tuning{};
@@ -159,15 +160,15 @@ struct sc_batch {
         return SC_OK;
     }
 
-    int build_items(uint32_t chunk) {
+    int build_items(uint32_t chunk, uint32_t warps) {
         std::vector<uint32_t> order(jobs.size());
         std::iota(order.begin(), order.end(), 0u);
         std::stable_sort(order.begin(), order.end(),
                          [&](uint32_t a, uint32_t b) { return jobs[a].n_photons > jobs[b].n_photons; });
         std::vector<WorkItem> items;
-        for (uint32_t j : order)
-            for (uint32_t b = 0; b < jobs[j].n_photons; b += chunk)
-                items.push_back(WorkItem{j, b, std::min(chunk, jobs[j].n_photons - b)});
+        uint64_t left = total_photons;
+        for (uint32_t j : order) cut_items(items, j, 0, jobs[j].n_photons, chunk, left, warps);
+        items_warps = warps;
         n_items = (uint32_t)items.size();
         if (d_items.n < items.size()) SC_CUDA(d_items.alloc(items.size()));
         if (!items.empty())
@@ -189,8 +190,9 @@ struct sc_batch {
         ff = any_free_flight();
         const int occ = batch_occupancy((int)n.aggregate, (int)n.minb, kBatchMaskWords, n.block, ff);
         grid = n.grid ? n.grid : (uint32_t)(ctx->sms * occ);
-        if (n.chunk_photons != tuning.chunk_photons || n_items == 0) {
-            int rc = build_items(n.chunk_photons);
+        const uint32_t warps = grid * (n.block / 32u);
+        if (n.chunk_photons != tuning.chunk_photons || warps != items_warps || n_items == 0) {
+            int rc = build_items(n.chunk_photons, warps);
             if (rc != SC_OK) return rc;
         }
         n.grid = grid;

@@ -388,10 +388,12 @@ struct sc_server {
         });
         const uint32_t chunk = cfg.chunk_photons;
         h_items.clear();
+        uint64_t left = 0;
+        for (const Request* q : active) left += q->r.job.n_photons;
         for (uint32_t i : order) {
             const Request* q = active[i];
-            const uint32_t N = q->r.job.n_photons, base = q->frame * N;
-            for (uint32_t b = 0; b < N; b += chunk) h_items.push_back(WorkItem{i, base + b, std::min(chunk, N - b)});
+            const uint32_t N = q->r.job.n_photons;
+            cut_items(h_items, i, q->frame * N, N, chunk, left, grid * 8u);
         }
         HostStage* h = nullptr;
         rc = stage_for((uint32_t)h_items.size(), &h);

@@ -96,3 +96,24 @@ def test_paths_through_several_solids(ctx, bounces):
         assert np.array_equal(states[i, :2 * k], st[:k].reshape(-1, 4)), i
     assert longest >= min(bounces, 5)
     f.close()
+
+
+@pytest.mark.parametrize("n_jobs,photons,chunk", [
+    (1, (1, 1), 0),               # one photon for all warps
+    (1, (200_000, 200_000), 64),  # items at their smallest
+    (3, (31, 70_001), 8192),      # shares far below the chunk
+    (40, (2_000, 500_000), 512),  # shares above the chunk, then below it
+    (2, (3_000_000, 3_000_000), 1 << 20)])
+def test_uneven_items_cover_every_photon(ctx, n_jobs, photons, chunk):
+    """Work items of any sizes trace each photon once: the batch's images equal
+    the plain per-scene launches' (which have no items)."""
+    from spectral_b200.batch import Batch, prism_jobs
+    jobs = prism_jobs(specs.random_prism_jobs(n_jobs, 3, 8, photons=photons, side=(40, 90)))
+    b = Batch(ctx, jobs, chunk_photons=chunk)
+    b.run()
+    b.synchronize()
+    batched = b.read_all_xyz()
+    b.run_plain()
+    b.synchronize()
+    assert np.array_equal(b.read_all_xyz(), batched)
+    b.close()
