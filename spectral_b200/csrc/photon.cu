@@ -449,6 +449,7 @@ cudaError_t launch_photons(const PhotonParams& p, const LaunchShape& shape, cuda
 // 201), 4 still win (prism 995 -> 464).
 static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk) {
     if (p.photon_count < (1u << 15)) return false;
+    if (8ull * chunk * 4ull * p.max_bounces > kCacheDeposits) return false;  // 8 warps, 4 samples a segment
     const f3 c = sub(add(p.corner, mul(add(p.bu, p.bv), 0.5f)), p.proj.o);
     const float depth = -dot(c, p.proj.w) / length(p.proj.w);
     const f3 across = cross(p.bdir, p.proj.w);  // on screen, square to the beam

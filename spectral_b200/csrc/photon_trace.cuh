@@ -81,7 +81,8 @@ __device__ __forceinline__ FilmView film_view(const PhotonParams& p, uint32_t bi
 // pixel, the one of a spectral film's pixel and bin) takes the slot its hash names
 // if that is free; others go straight to the film.  Sums are two 32-bit words per
 // value (12 low bits, and the rest), so that values below 2^23 stay exact over
-// 2^20 deposits, more than a CTA makes (8 warps x 256 photons x 64 bounces x 4).
+// kCacheDeposits deposits; launches whose CTAs could make more do without.
+constexpr uint64_t kCacheDeposits = 1u << 20;
 // V: values per cell.
 template <int V>
 struct CellCache {
@@ -528,7 +529,8 @@ __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& 
 template <bool SPEC>
 struct alignas(16) ParkedPhotons {
     float f[9][32];                // ox oy oz dx dy dz lambda power n(lambda)
-    uint32_t rng[32], meta[32];    // meta: bounce | glass of n + 1 << 8 | bin << 16
+    uint32_t rng[32], bounce[32];
+    uint32_t meta[32];             // glass of n + 1 (0: none yet) | bin << 16
     float c[SPEC ? 1 : 3][32];     // XYZ films: CMF of lambda
 };
 constexpr int kGroupLive = 24;
@@ -570,7 +572,8 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
                     park.f[3][q] = d.x; park.f[4][q] = d.y; park.f[5][q] = d.z;
                     park.f[6][q] = lambda; park.f[7][q] = power; park.f[8][q] = n_cached;
                     park.rng[q] = r.state;
-                    park.meta[q] = bounce | ((n_glass + 1u) << 8) | (bin << 16);
+                    park.bounce[q] = bounce;
+                    park.meta[q] = (n_glass <= 3u ? n_glass + 1u : 0u) | (bin << 16);
                     if (!SPEC) { park.c[0][q] = cx; park.c[SPEC ? 0 : 1][q] = cy; park.c[SPEC ? 0 : 2][q] = cz; }
                 }
                 parked += n;
@@ -601,8 +604,8 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
                     lambda = park.f[6][q]; power = park.f[7][q]; n_cached = park.f[8][q];
                     r.state = park.rng[q];
                     const uint32_t m = park.meta[q];
-                    bounce = m & 0xFFu;
-                    n_glass = ((m >> 8) & 0xFFu) - 1u;
+                    bounce = park.bounce[q];
+                    n_glass = (m & 0xFFFFu) - 1u;
                     bin = m >> 16;
                     if (!SPEC) { cx = park.c[0][q]; cy = park.c[SPEC ? 0 : 1][q]; cz = park.c[SPEC ? 0 : 2][q]; }
                     alive = true;

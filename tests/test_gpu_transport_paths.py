@@ -12,7 +12,7 @@ import pytest
 import oracle
 import spectral_b200 as sb
 from spectral_b200 import scenes, specs
-from helpers import axis_box, obeam, oscene
+from helpers import axis_box, device_desc, obeam, oscene
 
 pytestmark = pytest.mark.gpu
 
@@ -71,6 +71,33 @@ def test_one_launch_equals_many(ctx, name, w, h, bins, n, kw):
         f.dispatch_photons(a, min(a + 30_011, n), 5)
     assert whole.sum() > 0 and np.array_equal(f.read_raw(), whole)
     f.close()
+
+
+@pytest.mark.parametrize("bounces,n,part,bins", [
+    (300, 96, 1, 4),           # photons set aside after more than 255 bounces
+    (2000, 40_000, 4_000, 0)])  # more deposits of a CTA than the cell cache sums exactly
+def test_long_paths(ctx, bounces, n, part, bins):
+    """The device entry takes any bounce limit: photons totally reflected in a
+    glass cube until it, beside others that miss the cube, so that lanes fall idle
+    and photons of different bounces are set aside."""
+    import ctypes as C
+
+    import torch
+    from spectral_b200 import _lib
+    scene = sb.Scene(background=0.0)
+    scene.add_solid(axis_box((-1.0, -1.0, -1.0), (1.0, 1.0, 1.0)), sb.Dielectric(sb.SF11))
+    beam = sb.Beam((0.2, 0.0, 0.0), (1.4, 0.0, 0.0), (0.0, 0.01, 0.0), sb.f32_normalize((1.0, 1.0, 1.0)))
+    cam, keep, films = sb.Camera.look_at((0.0, 0.0, 8.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 40.0, 1.0), [], []
+    desc = device_desc(sb, _lib, torch, scene, cam, beam, 16, 16, 3, bins, keep)
+    desc.opts.max_bounces = bounces
+    for step in (n, part):
+        film = torch.zeros(_lib.lib.sc_film_bytes(16, 16, bins or 3) // 8, dtype=torch.int64, device="cuda")
+        for a in range(0, n, step):
+            _lib.check(_lib.lib.sc_trace_photons_device(ctx.h, C.byref(desc), a, min(step, n - a),
+                                                        C.c_void_p(film.data_ptr()), None, None))
+        torch.cuda.synchronize()
+        films.append(film)
+    assert films[0].sum().item() > 0 and torch.equal(films[0], films[1])
 
 
 @pytest.mark.parametrize("bounces", [1, 2, 8, 20])
