@@ -95,12 +95,24 @@ __host__ __device__ __forceinline__ float glass_n(uint32_t glass, float nm) {
 }
 
 // ---- sensor table lerp, clamped (spectral-core/src/cie.rs:47-61) ----------
+// Row position of a wavelength, (nm - 380) / 5 clamped to [0, 70] (NaN: 0).  On the
+// device the quotient is the product with 0.2f corrected by its fused remainder
+// (Brisebarre, Muller and Raina: division by a constant known in advance), which is
+// the rounded quotient for every mantissa; nm - 380 is 0 or at least 2^-15.
+__host__ __device__ __forceinline__ float tab_position(float nm) {
+    float x = nm - 380.0f;
+    if (!(x > 0.0f)) x = 0.0f;
+    if (x > 350.0f) x = 350.0f;
+#ifdef __CUDA_ARCH__
+    const float q = x * 0.2f;
+    return __fmaf_rn(__fmaf_rn(-5.0f, q, x), 0.2f, q);
+#else
+    return x / 5.0f;
+#endif
+}
 __host__ __device__ __forceinline__ float tab_sample(const float* col, float nm) {
-    float f = (nm - 380.0f) / 5.0f;
-    if (f < 0.0f) f = 0.0f;
-    if (f > (float)(kTableN - 1)) f = (float)(kTableN - 1);
-    if (f != f) f = 0.0f;
-    int i = (int)floorf(f);
+    const float f = tab_position(nm);
+    int i = (int)f;
     float frac = f - (float)i;
     if (i + 1 >= kTableN) return col[kTableN - 1];
     float a = col[i], b = col[i + 1];

@@ -9,16 +9,21 @@
 //             later rays as the next bounce reads them from the dense queue);
 //   shade     background / emission at termination, Fresnel / refract / TIR or
 //             Lambertian scatter, dispersion collapse to the hero lane, optional
-//             Russian roulette; survivors are compacted into the next queue with
-//             warp ballots, one atomic per block and shared-memory staging so the
-//             SoA writes are contiguous;
-//   tail      the few paths alive after the compacted bounces finish in one
-//             launch, kept compacted per CTA bounce by bounce;
+//             Russian roulette; each warp collects its survivors in shared memory
+//             and queues them 32 at a time;
+//   tail      the paths alive after the compacted bounces finish in one launch,
+//             idle lanes taking new paths from the queue;
 //   accumulate each pixel's samples summed in sample order (the CPU's order), so
 //             the image is deterministic and, for scenes without Lambertian
 //             surfaces, bit-identical to the CPU tracer.
 // Queue counts stay on the device: the launch sequence of an accumulate call is
 // fixed, needs no host synchronisation and is replayed from a CUDA graph.
+//
+// Bound: instruction issue (the stages' queues take 1 to 1.5 TB/s).  accumulate(64)
+// at 1280x720 of the prism on its floor 4.54 -> 3.05 ms, accumulate(4) at 333x187 of
+// glass under a sky 75 -> 54 us, from warps that compact and refill by themselves
+// (barriers were 30 to 60 % of the stage stalls), combs without radiance left out,
+// four table columns in one row, and quotients by constants as products.
 #include <algorithm>
 
 #include "internal.h"
@@ -29,16 +34,13 @@ namespace sc {
 namespace {
 
 constexpr int kShadeThreads = 256;
-// Shade and tail CTAs resident per SM: 5 (48 registers, small spills) hides
-// more of their queue-read and shared-memory latency than 4 (64 registers):
-// accumulate(64) at 1280x720 5.83 -> 5.37 ms; 6 or 8 tail CTAs spill more
-// and are slower again.
+// Shade and tail CTAs resident per SM: 5 (48 registers, small spills).
 constexpr int kStageCtasPerSm = 5;
 constexpr float kLambdaMin = 380.0f, kLambdaRange = 350.0f;
 
 struct TracerSmem {
     TracerParams p;
-    float tables[5 * kTableN];
+    float4 table[kTableN + 1];  // x, y, z and illuminant of a row; the last row twice
     sc_primitive prims[SC_MAX_PRIMS];
     sc_material mats[SC_MAX_PRIMS];
     float4 bounds[SC_MAX_PRIMS];
@@ -49,7 +51,12 @@ struct TracerSmem {
 __device__ __forceinline__ SceneView load_tracer(const TracerParams* gp, TracerSmem& s, sc_plane* planes) {
     const uint32_t tid = threadIdx.x;
     if (tid == 0) s.p = *gp;
-    for (uint32_t i = tid; i < 5u * kTableN; i += blockDim.x) s.tables[i] = gp->tables[i];
+    const float* tab = gp->tables;
+    const float* ill = tab + (gp->illuminant == 1u ? 4 : 3) * kTableN;
+    for (uint32_t i = tid; i <= (uint32_t)kTableN; i += blockDim.x) {
+        const uint32_t k = min(i, (uint32_t)kTableN - 1u);
+        s.table[i] = make_float4(tab[k], tab[kTableN + k], tab[2 * kTableN + k], ill[k]);
+    }
     __syncthreads();
     for (uint32_t i = tid; i < s.p.n_prims; i += blockDim.x) s.prims[i] = s.p.prims[i];
     for (uint32_t i = tid; i < s.p.n_mats; i += blockDim.x) s.mats[i] = s.p.mats[i];
@@ -62,41 +69,47 @@ __device__ __forceinline__ SceneView load_tracer(const TracerParams* gp, TracerS
 }
 
 __device__ __forceinline__ float lane_lambda(float u, int k) {
-    // SpectralSample::from_hero_u: (u*RANGE + k*RANGE/4).rem_euclid(RANGE).
-    // For 0 <= x < 2 RANGE (every u in [0, 1)) the remainder is x or x - RANGE,
-    // and x - RANGE is exact there (RANGE <= x < 2 RANGE), so it equals fmodf's
-    // exact remainder without its general loop.
+    // SpectralSample::from_hero_u: (u*RANGE + k*RANGE/4).rem_euclid(RANGE).  For
+    // 0 <= x < 2 RANGE (u is a draw, in [0, 1)) the remainder is x or x - RANGE,
+    // which is exact there (RANGE <= x < 2 RANGE).
     const float x = u * kLambdaRange + (float)k * (kLambdaRange / 4.0f);
-    float off;
-    if (x >= 0.0f && x < 2.0f * kLambdaRange) {
-        off = x >= kLambdaRange ? x - kLambdaRange : x;
-    } else {
-        off = fmodf(x, kLambdaRange);
-        if (off < 0.0f) off += kLambdaRange;
-    }
-    return kLambdaMin + off;
+    return kLambdaMin + (x >= kLambdaRange ? x - kLambdaRange : x);
+}
+
+// x / (1 / 350), correctly rounded: the product with the reciprocal (350 is that
+// of the rounded 1 / 350), corrected by its fused remainder (Brisebarre, Muller and
+// Raina, "Accelerating correctly rounded floating-point division when the divisor is
+// known in advance"; all mantissas compared with the quotient).  Where the
+// remainder could underflow or the product overflow: the division.
+__device__ __forceinline__ float over_pdf(float x) {
+    const float pdf = 1.0f / kLambdaRange;
+    if (!(x > 1e-25f && x < 1e25f)) return x / pdf;
+    const float q = x * kLambdaRange;
+    return __fmaf_rn(__fmaf_rn(-pdf, q, x), kLambdaRange, q);
 }
 
 // XYZ of a terminated comb whose lanes carry radiance rad_k = tp_k * e * S(lambda_k).
+// `valid`: 4 lanes, or 1 after a dispersive hit (dividing by either is scaling by
+// a power of two).  A comb of 1 lane has no radiance in the others: they are not
+// worked out (unless e is infinite: 0 * inf).  The four table columns lie in one
+// row, so a lane costs two 16-byte loads and one division by 5.
 __device__ __forceinline__ void comb_xyz(const TracerSmem& s, float u, float tp, uint32_t valid, float e,
                                          float out[3]) {
-    const float pdf = 1.0f / kLambdaRange;
-    const float* ill = s.tables + (s.p.illuminant == 1u ? 4 : 3) * kTableN;
-    // dividing by 1 or 4 lanes is scaling by a power of two: the same rounded
-    // quotient as the division
-    const bool pow2 = valid == 1u || valid == 4u;
-    const float inv_valid = valid == 4u ? 0.25f : 1.0f;
+    const bool one = valid == 1u;
+    const int lanes = one && fabsf(e) < __int_as_float(0x7f800000) ? 1 : 4;
+    const float inv_valid = one ? 1.0f : 0.25f;
     float x = 0.0f, y = 0.0f, z = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float lam = lane_lambda(u, k);
-        const float tk = (k == 0 || valid > 1u) ? tp : 0.0f;
-        const float rad = 0.0f + tk * e * tab_sample(ill, lam);
-        const float q = rad / pdf;
-        const float wk = pow2 ? q * inv_valid : q / (float)valid;
-        x += tab_sample(s.tables, lam) * wk;
-        y += tab_sample(s.tables + kTableN, lam) * wk;
-        z += tab_sample(s.tables + 2 * kTableN, lam) * wk;
+#pragma unroll 1
+    for (int k = 0; k < lanes; ++k) {
+        const float f = tab_position(lane_lambda(u, k));
+        const int i = (int)f;
+        const float frac = f - (float)i;
+        const float4 a = s.table[i], b = s.table[i + 1];
+        const float tk = k == 0 || !one ? tp : 0.0f;
+        const float wk = over_pdf(tk * e * (a.w + (b.w - a.w) * frac)) * inv_valid;
+        x += (a.x + (b.x - a.x) * frac) * wk;
+        y += (a.y + (b.y - a.y) * frac) * wk;
+        z += (a.z + (b.z - a.z) * frac) * wk;
     }
     out[0] = x; out[1] = y; out[2] = z;
 }
@@ -161,21 +174,30 @@ struct PathState {
     uint32_t rs, id, flags;  // RNG state, path id, valid lanes | depth << 8
 };
 
+__device__ __forceinline__ PathState read_path(const RayQueue& q, uint32_t i) {
+    PathState P;
+    P.o = mk(q.ox[i], q.oy[i], q.oz[i]);
+    P.d = mk(q.dx[i], q.dy[i], q.dz[i]);
+    P.tp = q.tp[i]; P.u = q.u[i]; P.rs = q.rng[i]; P.id = q.id[i]; P.flags = q.flags[i];
+    return P;
+}
+
 // Shade one path at `bounce` given its hit: background / emission ends the
-// path (its XYZ goes to result[id]); a surface scatters it (Fresnel / refract /
-// TIR or Lambertian, dispersion collapse, Russian roulette).  Returns whether
-// the path continues.
+// path (`lit`: with a radiance, in xyz; a path that meets none, as under a black
+// sky, has no comb to sum); a surface scatters it (Fresnel / refract / TIR or
+// Lambertian, dispersion collapse, Russian roulette).  Returns whether the path
+// continues.
 __device__ __forceinline__ bool shade_path(const TracerSmem& s, const SceneView& S, uint32_t bounce, PathState& P,
-                                           float t, f3 n, uint32_t info, float* result) {
+                                           float t, f3 n, uint32_t info, bool& lit, float xyz[3]) {
     const uint32_t kind = info >> 24;
     uint32_t valid = P.flags & 0xFFu;
+    lit = false;
     if (kind != 1u) {
         float e;
         if (kind == 0u) e = s.p.background + ((s.p.has_horizon && P.d.y > 0.0f) ? s.p.horizon : 0.0f);
         else e = s.p.em_scale;
-        float xyz[3];
-        comb_xyz(s, P.u, P.tp, valid, e, xyz);
-        result[3 * P.id] = xyz[0]; result[3 * P.id + 1] = xyz[1]; result[3 * P.id + 2] = xyz[2];
+        lit = e != 0.0f || !(fabsf(P.tp) < __int_as_float(0x7f800000));
+        if (lit) comb_xyz(s, P.u, P.tp, valid, e, xyz);
         return false;
     }
     const sc_material& m = S.mats[info & 0xFFFFu];
@@ -204,9 +226,43 @@ __device__ __forceinline__ bool shade_path(const TracerSmem& s, const SceneView&
     return survive;
 }
 
-// One compacted bounce: each path's ray is intersected and shaded here, and
-// the survivors are compacted into the next ray queue (no hit queue: the
-// bounce that reads a ray intersects it, from the dense queue).
+// n / d and its remainder for a d whose `inv` = floor((2^32 - 1) / d) is known: the
+// high word of n * inv is the quotient or one less.
+struct FastDiv {
+    uint32_t d, inv;
+    __device__ __forceinline__ explicit FastDiv(uint32_t v) : d(v), inv(0xFFFFFFFFu / v) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t n, uint32_t& rem) const {
+        uint32_t q = __umulhi(n, inv);
+        rem = n - q * d;
+        if (rem >= d) { ++q; rem -= d; }
+        return q;
+    }
+};
+
+// Survivors of a warp on their way into the next ray queue: a ring of 64 in shared
+// memory.  Full groups of 32 go out with one atomic and whole 128-byte lines, and
+// no warp waits for another one of its CTA (compacting per CTA cost three barriers
+// a bounce: 30 % of the stalls).
+struct PathRing {
+    float f[8][64];
+    uint32_t u[3][64];
+};
+__device__ __forceinline__ void ring_write(const PathRing& ring, uint32_t head, uint32_t n, const RayQueue& out,
+                                           uint32_t* count, uint32_t lane) {
+    uint32_t g = 0;
+    if (lane == 0) g = atomicAdd(count, n);
+    g = __shfl_sync(0xffffffffu, g, 0) + lane;
+    if (lane >= n) return;
+    const uint32_t j = (head + lane) & 63u;
+    out.ox[g] = ring.f[0][j]; out.oy[g] = ring.f[1][j]; out.oz[g] = ring.f[2][j];
+    out.dx[g] = ring.f[3][j]; out.dy[g] = ring.f[4][j]; out.dz[g] = ring.f[5][j];
+    out.tp[g] = ring.f[6][j]; out.u[g] = ring.f[7][j];
+    out.rng[g] = ring.u[0][j]; out.id[g] = ring.u[1][j]; out.flags[g] = ring.u[2][j];
+}
+
+// One compacted bounce: each path's ray is intersected and shaded here, and the
+// survivors are compacted into the next ray queue (no hit queue: the bounce that
+// reads a ray intersects it, from the dense queue).
 // GEN: the first bounce with no queue in: each path's primary ray is made here
 // (stream key mix2(pixel, sample index), jittered through the pixel, hero-comb
 // draw), intersected in place and shaded.  Paths of a wave are numbered
@@ -220,160 +276,125 @@ __global__ void __launch_bounds__(kShadeThreads, kStageCtasPerSm) tr_shade(const
                                                           uint32_t n_pixels, uint32_t n_paths,
                                                           const uint32_t* __restrict__ base) {
     __shared__ TracerSmem s;
-    __shared__ uint32_t warp_base[kShadeThreads / 32 + 1];
-    __shared__ uint32_t block_base;
-    __shared__ float st_f[8][kShadeThreads];      // staged survivors: ox oy oz dx dy dz tp u
-    __shared__ uint32_t st_u[3][kShadeThreads];   // rng id flags
+    __shared__ PathRing rings[kShadeThreads / 32];
     extern __shared__ __align__(16) unsigned char dyn[];
     if (GEN && blockIdx.x == 0 && threadIdx.x == 0) counts[0] = n_paths;
     const uint32_t n = GEN ? n_paths : counts[bounce];
     if (blockIdx.x * blockDim.x >= n) return;  // nothing queued for this CTA (late bounces)
     const SceneView S = load_tracer(gp, s, reinterpret_cast<sc_plane*>(dyn));
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    PathRing& ring = rings[threadIdx.x >> 5];
     const uint32_t b0 = GEN ? *base : 0u;
-    for (uint32_t tile = blockIdx.x * blockDim.x; tile < n; tile += gridDim.x * blockDim.x) {
-        const uint32_t i = tile + threadIdx.x;
-        bool survive = false;
+    const FastDiv per_sample(n_pixels), per_row(s.p.width);
+    uint32_t head = 0, held = 0;  // the same in every lane
+    for (uint32_t tile = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); tile < n; tile += gridDim.x * blockDim.x) {
+        const uint32_t i = tile + lane;
+        bool survive = false, lit = false;
         PathState P;
-        P.o = P.d = mk(0.0f, 0.0f, 0.0f);
-        P.tp = P.u = 0.0f;
-        P.rs = P.id = P.flags = 0u;
-        if (i < n && GEN) {
-            const uint32_t smp = i / n_pixels, pixel = first_pixel + (i - smp * n_pixels);
-            const uint32_t px = pixel % s.p.width, py = pixel / s.p.width;
-            Rng r = Rng::make(mix2(pixel, b0 + smp), s.p.seed);
-            const float fs = ((float)px + r.f32()) / (float)s.p.width;
-            const float ft = 1.0f - ((float)py + r.f32()) / (float)s.p.height;
-            P.u = r.f32();
-            P.o = ld3(s.p.cam.origin);
-            P.d = primary_dir(s.p.cam, fs, ft);
-            P.rs = r.state; P.tp = 1.0f; P.id = i; P.flags = 4u;
-            result[3 * i] = 0.0f; result[3 * i + 1] = 0.0f; result[3 * i + 2] = 0.0f;
+        float xyz[3] = {0.0f, 0.0f, 0.0f};
+        if (i < n) {
+            if (GEN) {
+                uint32_t j, px;
+                const uint32_t smp = per_sample(i, j), pixel = first_pixel + j, py = per_row(pixel, px);
+                Rng r = Rng::make(mix2(pixel, b0 + smp), s.p.seed);
+                const float fs = ((float)px + r.f32()) / (float)s.p.width;
+                const float ft = 1.0f - ((float)py + r.f32()) / (float)s.p.height;
+                P.u = r.f32();
+                P.o = ld3(s.p.cam.origin);
+                P.d = primary_dir(s.p.cam, fs, ft);
+                P.rs = r.state; P.tp = 1.0f; P.id = i; P.flags = 4u;
+            } else {
+                P = read_path(q, i);
+            }
             float t;
             f3 nrm;
             uint32_t info;
             trace_hit(s, S, P.o, P.d, t, nrm, info);
-            if ((info >> 24) != 1u) nrm = mk(0.0f, 0.0f, 0.0f);
-            survive = shade_path(s, S, 0u, P, t, nrm, info, result);
-        } else if (i < n) {
-            P.o = mk(q.ox[i], q.oy[i], q.oz[i]);
-            P.d = mk(q.dx[i], q.dy[i], q.dz[i]);
-            P.tp = q.tp[i]; P.u = q.u[i]; P.rs = q.rng[i]; P.id = q.id[i]; P.flags = q.flags[i];
-            float t;
-            f3 nrm;
-            uint32_t info;
-            trace_hit(s, S, P.o, P.d, t, nrm, info);
-            if ((info >> 24) != 1u) nrm = mk(0.0f, 0.0f, 0.0f);
-            survive = shade_path(s, S, bounce, P, t, nrm, info, result);
+            survive = shade_path(s, S, GEN ? 0u : bounce, P, t, nrm, info, lit, xyz);
+            if (GEN || lit) {
+                float* o = result + 3 * (size_t)P.id;
+                o[0] = xyz[0]; o[1] = xyz[1]; o[2] = xyz[2];
+            }
         }
-        const f3 o = P.o, d = P.d;
-        const float tp = P.tp, u = P.u;
-        const uint32_t rs = P.rs, id = P.id, flags = P.flags;
-        // block-level compaction: ballot per warp, prefix over warps, one atomic
         const unsigned ball = __ballot_sync(0xffffffffu, survive);
-        const uint32_t rank = __popc(ball & ((1u << lane) - 1u));
-        if (lane == 0) warp_base[warp] = __popc(ball);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t acc = 0;
-            for (int w = 0; w < kShadeThreads / 32; ++w) { const uint32_t c = warp_base[w]; warp_base[w] = acc; acc += c; }
-            warp_base[kShadeThreads / 32] = acc;
-            block_base = acc ? atomicAdd(&counts[bounce + 1], acc) : 0u;
-        }
-        __syncthreads();
         if (survive) {
-            const uint32_t j = warp_base[warp] + rank;
-            st_f[0][j] = o.x; st_f[1][j] = o.y; st_f[2][j] = o.z;
-            st_f[3][j] = d.x; st_f[4][j] = d.y; st_f[5][j] = d.z;
-            st_f[6][j] = tp; st_f[7][j] = u;
-            st_u[0][j] = rs; st_u[1][j] = id; st_u[2][j] = flags;
+            const uint32_t j = (head + held + __popc(ball & ((1u << lane) - 1u))) & 63u;
+            ring.f[0][j] = P.o.x; ring.f[1][j] = P.o.y; ring.f[2][j] = P.o.z;
+            ring.f[3][j] = P.d.x; ring.f[4][j] = P.d.y; ring.f[5][j] = P.d.z;
+            ring.f[6][j] = P.tp; ring.f[7][j] = P.u;
+            ring.u[0][j] = P.rs; ring.u[1][j] = P.id; ring.u[2][j] = P.flags;
         }
-        __syncthreads();
-        const uint32_t total = warp_base[kShadeThreads / 32];
-        if (threadIdx.x < total) {
-            const uint32_t j = threadIdx.x, g = block_base + j;
-            out.ox[g] = st_f[0][j]; out.oy[g] = st_f[1][j]; out.oz[g] = st_f[2][j];
-            out.dx[g] = st_f[3][j]; out.dy[g] = st_f[4][j]; out.dz[g] = st_f[5][j];
-            out.tp[g] = st_f[6][j]; out.u[g] = st_f[7][j];
-            out.rng[g] = st_u[0][j]; out.id[g] = st_u[1][j]; out.flags[g] = st_u[2][j];
+        held += __popc(ball);
+        __syncwarp();
+        if (held >= 32u) {
+            ring_write(ring, head, 32u, out, counts + bounce + 1, lane);
+            head += 32u;
+            held -= 32u;
+            __syncwarp();
         }
-        __syncthreads();
     }
+    if (held) ring_write(ring, head, held, out, counts + bounce + 1, lane);
 }
 
-// Late bounces: by the third bounce only a few per cent of a wave's paths are
-// alive, and a launch pair per bounce costs more than the work.  The tail runs
-// them in one launch: each CTA holds up to 256 paths in shared memory with the
-// live ones at the front, runs one bounce of all of them (the same hit and
-// shade code, so the image is unchanged), compacts the survivors with warp
-// ballots, and refills the free slots from the queue with one claim per CTA
-// (counter counts[max_depth + 1], zero at entry), so its warps stay full while
-// the paths end after different numbers of bounces.  Segments after each
-// path's first tail bounce are added to counts[first + 1].
+// The bounces after the compacted ones in one launch: each lane keeps a path in
+// registers until it ends, and a warp with fewer than kTailLive paths claims new
+// ones from the queue for its idle lanes (counter counts[max_depth + 1], zero
+// at entry), whatever bounces the others are at.  Warps
+// stay full without waiting for one another.  The same hit and shade code, so the
+// image is unchanged.  Segments after each path's first tail bounce are added to
+// counts[first + 1].
+constexpr uint32_t kTailLive = 24;
 __global__ void __launch_bounds__(256, kStageCtasPerSm) tr_tail(const TracerParams* __restrict__ gp, uint32_t first,
                                                                 RayQueue q, uint32_t* counts, float* result) {
     __shared__ TracerSmem s;
-    __shared__ float sf[8][256];    // ox oy oz dx dy dz tp u
-    __shared__ uint32_t su[3][256]; // rng id flags
-    __shared__ uint32_t warp_base[8 + 1];
-    __shared__ uint32_t claim_base;
     extern __shared__ __align__(16) unsigned char dyn[];
     const uint32_t n = counts[first];
     if (blockIdx.x * blockDim.x >= n) return;
     const SceneView S = load_tracer(gp, s, reinterpret_cast<sc_plane*>(dyn));
     uint32_t* claim = counts + s.p.max_depth + 1;
-    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    uint32_t live = 0, segs = 0;
+    const uint32_t lane = threadIdx.x & 31u;
+    // A claim is a quarter of a warp's share, 32 to 256 paths: one per refill made the
+    // warps queue up at the counter (all bounces but the first here, 1280x720, 64 spp:
+    // 4.29 ms).
+    const uint32_t share = n / (4u * gridDim.x * (blockDim.x >> 5));
+    const uint32_t step = share < 32u ? 32u : share > 256u ? 256u : share & ~31u;
+    uint32_t segs = 0, next = 0, end = 0;  // next, end: what is left of the claim, the same in every lane
+    bool alive = false, more = true;
+    PathState P;
     for (;;) {
-        if (t == 0) claim_base = atomicAdd(claim, 256u - live);
-        __syncthreads();
-        const uint32_t base = claim_base;
-        const uint32_t got = base >= n ? 0u : min(256u - live, n - base);
-        if (t >= live && t < live + got) {  // coalesced: consecutive slots take consecutive paths
-            const uint32_t i = base + (t - live);
-            sf[0][t] = q.ox[i]; sf[1][t] = q.oy[i]; sf[2][t] = q.oz[i];
-            sf[3][t] = q.dx[i]; sf[4][t] = q.dy[i]; sf[5][t] = q.dz[i];
-            sf[6][t] = q.tp[i]; sf[7][t] = q.u[i];
-            su[0][t] = q.rng[i]; su[1][t] = q.id[i]; su[2][t] = q.flags[i];
+        const unsigned live = __ballot_sync(0xffffffffu, alive);
+        const uint32_t m = __popc(live);
+        if (more && m < kTailLive) {
+            if (next == end) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(claim, step);
+                next = min(__shfl_sync(0xffffffffu, at, 0), n);
+                end = next + min(step, n - next);
+                more = next < n;
+            }
+            const uint32_t i = next + __popc(~live & ((1u << lane) - 1u));
+            if (!alive && i < end) {
+                P = read_path(q, i);
+                alive = true;
+            }
+            next = min(next + 32u - m, end);
+        } else if (m == 0u) {
+            break;
         }
-        live += got;
-        __syncthreads();
-        if (live == 0) break;
-        bool survive = false;
-        PathState P;
-        P.o = P.d = mk(0.0f, 0.0f, 0.0f);
-        P.tp = P.u = 0.0f;
-        P.rs = P.id = P.flags = 0u;
-        if (t < live) {
-            P.o = mk(sf[0][t], sf[1][t], sf[2][t]);
-            P.d = mk(sf[3][t], sf[4][t], sf[5][t]);
-            P.tp = sf[6][t]; P.u = sf[7][t]; P.rs = su[0][t]; P.id = su[1][t]; P.flags = su[2][t];
+        if (alive) {
             const uint32_t b = (P.flags >> 8) & 0xFFu;  // the bounce this path is at
-            float th;
+            float t, xyz[3];
             f3 nrm;
             uint32_t info;
-            trace_hit(s, S, P.o, P.d, th, nrm, info);
+            bool lit;
+            trace_hit(s, S, P.o, P.d, t, nrm, info);
             if (b > first) ++segs;  // counts[first] already holds the first tail bounce's rays
-            survive = shade_path(s, S, b, P, th, nrm, info, result);
+            alive = shade_path(s, S, b, P, t, nrm, info, lit, xyz);
+            if (lit) {
+                float* o = result + 3 * (size_t)P.id;
+                o[0] = xyz[0]; o[1] = xyz[1]; o[2] = xyz[2];
+            }
         }
-        const unsigned ball = __ballot_sync(0xffffffffu, survive);
-        if (lane == 0) warp_base[warp] = __popc(ball);
-        __syncthreads();  // every slot has been read
-        if (t == 0) {
-            uint32_t acc = 0;
-            for (int w = 0; w < 8; ++w) { const uint32_t c = warp_base[w]; warp_base[w] = acc; acc += c; }
-            warp_base[8] = acc;
-        }
-        __syncthreads();
-        if (survive) {
-            const uint32_t j = warp_base[warp] + __popc(ball & ((1u << lane) - 1u));
-            sf[0][j] = P.o.x; sf[1][j] = P.o.y; sf[2][j] = P.o.z;
-            sf[3][j] = P.d.x; sf[4][j] = P.d.y; sf[5][j] = P.d.z;
-            sf[6][j] = P.tp; sf[7][j] = P.u;
-            su[0][j] = P.rs; su[1][j] = P.id; su[2][j] = P.flags;
-        }
-        live = warp_base[8];
-        __syncthreads();  // the survivors are in place (and warp_base is read) before the next claim
     }
     for (int o = 16; o > 0; o >>= 1) segs += __shfl_xor_sync(0xffffffffu, segs, o);
     if (lane == 0 && segs) atomicAdd(counts + first + 1, segs);
@@ -439,7 +460,11 @@ cudaError_t launch_tracer_wave(const TracerParams* d_params, const TracerLaunch&
     const size_t dyn = tracer_dyn_smem(L.n_planes);
     // wavefront with compaction for the first bounces, then the tail in place;
     // the first bounce makes, intersects and shades the primary rays in one kernel
-    const uint32_t wave_bounces = L.max_depth < L.wave_bounces ? L.max_depth : L.wave_bounces;
+    // (where the caller does not say: two, or one for waves that the tail's warps
+    // hold with few refills.  accumulate(64) at 1280x720, waves of 2^22 paths: one 3.28
+    // ms, two 3.05, three 3.06; accumulate(4) at 333x187: 54, 60, 64 us)
+    const uint32_t want = L.wave_bounces ? L.wave_bounces : n_paths <= (1u << 20) ? 1u : 2u;
+    const uint32_t wave_bounces = L.max_depth < want ? L.max_depth : want;
     // bounce b intersects and shades the rays of bounce b and queues its
     // compacted survivors (ray queues alternate)
     for (uint32_t b = 0; b < wave_bounces; ++b) {

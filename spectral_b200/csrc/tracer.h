@@ -36,7 +36,7 @@ struct TracerLaunch {
     const uint32_t* d_base; // sample index of the first sample of this accumulate
     unsigned long long* segments;  // running count of traced segments
     uint32_t spp, max_depth, n_planes, grid;
-    uint32_t wave_bounces;  // compacted wavefront bounces before the tail
+    uint32_t wave_bounces;  // compacted wavefront bounces before the tail (0: by the wave's size)
 };
 
 // out[i] = sum[i] / count for the n floats of the running sums.

@@ -13,16 +13,11 @@
 using namespace sc;
 
 namespace {
-// Waves run on chains (one stream and one queue set each), so one wave's short
-// late-bounce launches overlap other waves' full-width ones.  Measured on the
-// 1280x720, 64 spp workload (accumulate(64)): 2 chains of 2^19-path waves
-// (queues in L2) 7.47 ms, 3 x 2^20 6.39 ms, 3 x 2^22 6.11 ms, 2 x 2^24
-// 6.14 ms: large waves give the in-place tail enough paths to fill the GPU, and
-// the stages are bound by latency and issue, not by the queues' DRAM traffic.
-// With the first shade making its own rays and 5 stage CTAs per SM: 2 x 2^22
-// 5.52 ms, 3 x 2^21 5.47, 3 x 2^22 5.39, 4 x 2^23 5.35 (within run-to-run
-// spread of 3 x 2^22); two compacted bounces before the tail stay best (one
-// 6.45, three 5.75, four 5.67 ms).
+// Waves run on chains (one stream and one queue set each), so one wave's late
+// bounces overlap other waves' full-width ones.  accumulate(64) at 1280x720: 3 chains
+// of 2^20-path waves 4.21 ms, 2^21 3.59, 2^22 3.28, 2^23 3.21; 1 x 2^24 3.56, 2 x 2^22
+// 3.38, 4 x 2^22 3.28 (one compacted bounce): large waves fill the GPU, and the
+// stages are bound by issue, not by the queues' DRAM traffic.
 constexpr uint32_t kMaxChains = 4;
 constexpr uint32_t kDefaultChains = 3;
 constexpr uint32_t kDefaultWaveLog2 = 22;  // paths per wave and chain: 2^22
@@ -235,7 +230,7 @@ int sc_tracer_create(sc_ctx* ctx, const sc_primitive* prims, uint32_t n_prims, c
         L.counts = t->counts.p + c * (o.max_depth + 2); L.sum = t->sum.p; L.d_base = t->base.p;
         L.segments = t->segments.p;
         L.max_depth = o.max_depth; L.n_planes = n_planes; L.grid = (uint32_t)tracer_grid(ctx->sms);
-        L.wave_bounces = o.wave_bounces ? o.wave_bounces : 2u;
+        L.wave_bounces = o.wave_bounces;
     }
     if ((e = cudaMemcpy(t->params.p, &hp, sizeof hp, cudaMemcpyHostToDevice)) != cudaSuccess) return fail(e);
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail(e);
