@@ -282,13 +282,13 @@ __device__ __forceinline__ uint32_t beam_step(const PhotonParams& p, uint32_t* s
 template <bool SPEC>
 __device__ __forceinline__ void deposit_pixel(const PhotonParams& p, uint32_t px, uint32_t py, const StepRec& R,
                                               float w) {
-    unsigned long long* c = p.film + film_cell(px, py, p.tiles_x, p.channels);
+    unsigned long long* c = p.film + film_cell(px, py, p.tiles_x, SPEC ? p.channels : 3u, SPEC ? R.bin : 0u);
     if (SPEC) {
-        red_u64(c + R.bin, fixed_scaled(R.c0[0] * w));
+        red_u64(c, fixed_scaled(R.c0[0] * w));
     } else {
         red_u64(c, fixed_scaled(R.c0[0] * w));
-        red_u64(c + 1, fixed_scaled(R.c1[0] * w));
-        red_u64(c + 2, fixed_scaled(R.c2[0] * w));
+        red_u64(c + kTilePixels, fixed_scaled(R.c1[0] * w));
+        red_u64(c + 2 * kTilePixels, fixed_scaled(R.c2[0] * w));
     }
 }
 
@@ -334,10 +334,10 @@ __device__ __forceinline__ void window_march(const PhotonParams& p, const BeamWa
 #pragma unroll
         for (int c = 0; c < CH; ++c) any |= acc[k][c] != bias;
         if (any) {
-            unsigned long long* cell = p.film + film_cell(px, py[k], p.tiles_x, p.channels) + (SPEC ? bin : 0u);
+            unsigned long long* cell = p.film + film_cell(px, py[k], p.tiles_x, SPEC ? p.channels : 3u, SPEC ? bin : 0u);
 #pragma unroll
             for (int c = 0; c < CH; ++c) {
-                atomicAdd(cell + c, (unsigned long long)(acc[k][c] - bias));
+                atomicAdd(cell + c * kTilePixels, (unsigned long long)(acc[k][c] - bias));
                 acc[k][c] = bias;
             }
         }

@@ -594,8 +594,8 @@ int sc_photon_film_read_raw(sc_photon_film* f, int64_t* out) {
     const FilmGeom& g = f->geom;
     for (uint32_t py = 0; py < g.h; ++py)
         for (uint32_t px = 0; px < g.w; ++px)
-            std::memcpy(out + ((size_t)py * g.w + px) * g.channels, tiles.data() + film_cell(px, py, g.tiles_x, g.channels),
-                        g.channels * sizeof(int64_t));
+            for (uint32_t c = 0; c < g.channels; ++c)
+                out[((size_t)py * g.w + px) * g.channels + c] = tiles[film_cell(px, py, g.tiles_x, g.channels, c)];
     return SC_OK;
     SC_GUARD_END
 }

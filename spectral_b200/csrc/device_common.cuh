@@ -296,17 +296,29 @@ __device__ __forceinline__ unsigned long long to_fixed(float x, float scale) {
     return (unsigned long long)__float2ll_rn(y);
 }
 
-// Film layout: 8x8-pixel tiles, tile-major, `channels` int64 per pixel.
+// Film layout: 8x8-pixel tiles, tile-major; inside a tile channel-major, and the
+// 64 pixels of a channel so that neighbours in a row or a column lie in different
+// 128-byte lines (pixel (x, y) in line (x + y) mod 4).  L2 adds to one line a few times
+// slower than to several, and photons of all wavelengths meet in the pixels of a
+// narrow beam, whose cells side by side were a few lines.  Pixel by pixel against
+// this: prism, 2^20 photons at 640x360: 16 bins 261 -> 175 us, 64 bins 200 -> 175, XYZ
+// 472 -> 379; 900,000 photons at 200x190: 16 bins 388 -> 239, 32 bins 333 -> 165.
+// (Channel-major with the pixels in reading order: 16 bins 193 and 255, XYZ 472.)
 __host__ __device__ __forceinline__ uint32_t film_tile(uint32_t px, uint32_t py, uint32_t tiles_x) {
     return (py >> kTileShift) * tiles_x + (px >> kTileShift);
 }
-// The pixel's index in tile-major order fits 32 bits (every entry point limits
-// a film to 2^28 pixels, and beam films to 65535 x 65535: at most 2^26 tiles of
-// 64 pixels), so it is formed in 32-bit integer arithmetic and widened once, by
-// the multiply with the channel count.
-__host__ __device__ __forceinline__ size_t film_cell(uint32_t px, uint32_t py, uint32_t tiles_x, uint32_t channels) {
-    const uint32_t local = ((py & 7u) << 3) | (px & 7u);
-    return (size_t)((film_tile(px, py, tiles_x) << 6) | local) * channels;
+// Position of a pixel among the 64 of its tile, and the pixel (y << 3 | x) at one.
+__host__ __device__ __forceinline__ uint32_t film_local(uint32_t px, uint32_t py) {
+    return (((px + py) & 3u) << 4) | ((py & 7u) << 1) | ((px >> 2) & 1u);
+}
+__host__ __device__ __forceinline__ uint32_t film_local_pixel(uint32_t at) {
+    const uint32_t y = (at >> 1) & 7u;
+    return (y << 3) | ((at & 1u) << 2) | (((at >> 4) - y) & 3u);
+}
+// Films have at most 2^28 pixels (beam films 65535 x 65535): below 2^26 tiles.
+__host__ __device__ __forceinline__ size_t film_cell(uint32_t px, uint32_t py, uint32_t tiles_x, uint32_t channels,
+                                                     uint32_t channel = 0) {
+    return (size_t)film_tile(px, py, tiles_x) * (kTilePixels * channels) + channel * kTilePixels + film_local(px, py);
 }
 
 }  // namespace sc

@@ -88,24 +88,26 @@ __device__ __forceinline__ void reduce_staged(const TileRef& t, bool drain, cons
             const uint32_t px = tx * 8u + (l & 7u), py = ty * 8u + (l >> 3);
             if (px < p.width && py < p.height)
                 p.xyz[((size_t)py * p.width + px) * 3u + c] =
-                    t.dirty ? (float)((double)(long long)sm[i] * p.inv_scale) : 0.0f;
+                    t.dirty ? (float)((double)(long long)sm[c * (uint32_t)kTilePixels + film_local(l, l >> 3)] *
+                                      p.inv_scale)
+                            : 0.0f;
         }
     } else {
-        // 4 threads per pixel, each a contiguous quarter of the bins; partials
-        // are summed in quarter order so the result does not depend on timing.
+        // 4 threads per pixel, each a contiguous quarter of the bins (a warp reads 32
+        // cells of one bin side by side); partials are summed in quarter order so the result does
+        // not depend on timing.
         const uint32_t l = tid & 63u, q = tid >> 6;
         if (q < 4u) {
-            const uint32_t b0 = q * C / 4u, b1 = (q + 1u) * C / 4u, span = b1 - b0;
+            const uint32_t b0 = q * C / 4u, b1 = (q + 1u) * C / 4u;
             double x = 0.0, y = 0.0, z = 0.0;
-            const unsigned long long* row = sm + (size_t)l * C;
-            for (uint32_t j = 0; j < span; ++j) {
-                const uint32_t b = b0 + (j + l) % span;  // rotate to spread banks
-                const double v = (double)(long long)row[b];
+            for (uint32_t b = b0; b < b1; ++b) {
+                const double v = (double)(long long)sm[b * (uint32_t)kTilePixels + l];
                 x += v * (double)p.binw[b];
                 y += v * (double)p.binw[C + b];
                 z += v * (double)p.binw[2u * C + b];
             }
-            part[(q * 64u + l) * 3u] = x; part[(q * 64u + l) * 3u + 1u] = y; part[(q * 64u + l) * 3u + 2u] = z;
+            double* o = part + (q * 64u + film_local_pixel(l)) * 3u;
+            o[0] = x; o[1] = y; o[2] = z;
         }
         __syncthreads();
         if (tid < 64u) {

@@ -152,12 +152,11 @@ __global__ void rng_draws_kernel(uint32_t key, uint32_t seed, uint32_t n, uint32
 }
 
 // ---------------------------------------------------------------------------
-// Wavelength-ordered dispatch.  Film cells are pixel-major (the bins of a pixel
-// are adjacent), so photons of random wavelengths traced together touch every
-// 32-byte sector of every pixel they reach, and a spectral film larger than L2
-// misses on most of its atomics.  Tracing the photons of a launch in order of
-// their film bin keeps the photons in flight within a few bins: about one
-// sector per pixel is live at a time.  The photons and their paths are the
+// Wavelength-ordered dispatch.  Photons of random wavelengths traced together
+// touch the sectors of all bins of every pixel they reach, and a spectral film
+// larger than L2 misses on most of its atomics.  Tracing the photons of a launch
+// in order of their film bin keeps the photons in flight within a few bins: a few
+// sectors for every four pixels are live at a time.  The photons and their paths are the
 // same and the film is a sum of exact integers, so the image is bit-identical.
 // Counting sort of the launch's photons by key (kOrderKeys groups of
 // consecutive bins): per-CTA key histograms of contiguous photon chunks

@@ -59,16 +59,21 @@ __device__ __forceinline__ void mark_tile(const PhotonParams& p, uint32_t* smask
     }
 }
 
-// Film access of one photon: its bin's cell of pixel 0, the bytes from pixel to
-// pixel, tiles per row.
+// Film access of one photon: its bin's cells of tile 0, the cells of a tile, tiles
+// per row.
 struct FilmView {
     unsigned long long* cell0;
-    uint32_t stride, tiles_x;
+    uint32_t tile_cells, tiles_x;
+    // `pixel`: tile << 6 | film_local()
+    __device__ __forceinline__ unsigned long long* cell(uint32_t pixel) const {
+        return cell0 + (size_t)(pixel >> 6) * tile_cells + (pixel & 63u);
+    }
 };
+template <bool SPEC>
 __device__ __forceinline__ FilmView film_view(const PhotonParams& p, uint32_t bin) {
     FilmView v;
-    v.cell0 = p.film + bin;
-    v.stride = p.channels * 8u;
+    v.cell0 = p.film + (SPEC ? bin * kTilePixels : 0u);
+    v.tile_cells = (SPEC ? p.channels : 3u) * kTilePixels;
     v.tiles_x = p.tiles_x;
     return v;
 }
@@ -88,7 +93,7 @@ template <int V>
 struct CellCache {
     static constexpr uint32_t kLog2 = V == 3 ? 11u : 12u, kSlots = 1u << kLog2;
     static constexpr uint32_t kFree = 0xFFFFFFFFu;
-    uint32_t key[kSlots];         // pixel (tile-major) x cells of a pixel + bin, or free
+    uint32_t key[kSlots];         // the cell's position in the film (XYZ: its pixel, tile-major), or free
     uint32_t sum[2 * V][kSlots];  // low and high words of the values
     __device__ __forceinline__ void clear() {
         for (uint32_t i = threadIdx.x; i < kSlots; i += blockDim.x) {
@@ -97,14 +102,15 @@ struct CellCache {
             for (int k = 0; k < 2 * V; ++k) sum[k][i] = 0u;
         }
     }
-    // Adds the sums to the film; key k is V-tuple k of its cells.
+    // Adds the sums to the film.
     __device__ __forceinline__ void flush(unsigned long long* film) const {
         for (uint32_t i = threadIdx.x; i < kSlots; i += blockDim.x) {
             if (key[i] == kFree) continue;
-            unsigned long long* cell = film + (size_t)key[i] * V;
+            unsigned long long* cell = V == 1 ? film + key[i]
+                                              : film + (size_t)(key[i] >> 6) * (V * kTilePixels) + (key[i] & 63u);
 #pragma unroll
             for (int k = 0; k < V; ++k)
-                red_u64(cell + k, (unsigned long long)sum[2 * k][i] + ((unsigned long long)sum[2 * k + 1][i] << 12));
+                red_u64(cell + k * kTilePixels, (unsigned long long)sum[2 * k][i] + ((unsigned long long)sum[2 * k + 1][i] << 12));
         }
     }
     // Whether the values went into the cache.
@@ -133,9 +139,10 @@ constexpr uint32_t kCacheBins = 8;
 template <bool SPEC> using CellCacheOf = CellCache<SPEC ? 1 : 3>;
 
 template <bool SPEC>
-__device__ __forceinline__ bool cache_take(CellCacheOf<SPEC>& cache, const PhotonParams& p, uint32_t pixel, uint32_t bin,
-                                           unsigned long long v0, unsigned long long v1, unsigned long long v2) {
-    if constexpr (SPEC) return cache.add(pixel * p.channels + bin, {v0});
+__device__ __forceinline__ bool cache_take(CellCacheOf<SPEC>& cache, const PhotonParams& p, uint32_t pixel,
+                                           const unsigned long long* cell, unsigned long long v0,
+                                           unsigned long long v1, unsigned long long v2) {
+    if constexpr (SPEC) return cache.add((uint32_t)(cell - p.film), {v0});  // below 2^31: kCacheBins
     else return cache.add(pixel, {v0, v1, v2});
 }
 
@@ -145,14 +152,14 @@ __device__ __forceinline__ bool cache_take(CellCacheOf<SPEC>& cache, const Photo
 template <bool SPEC, int AGG>
 __device__ __forceinline__ void deposit(const PhotonParams& p, const FilmView& fv, uint32_t* smask, bool ok,
                                         uint32_t px, uint32_t py, float contrib, float cx, float cy, float cz,
-                                        float scale, CellCacheOf<SPEC>* cache = nullptr, uint32_t bin = 0) {
+                                        float scale, CellCacheOf<SPEC>* cache = nullptr) {
     unsigned long long* cell = nullptr;
     uint32_t tile = 0, pixel = 0;
     unsigned long long v0 = 0, v1 = 0, v2 = 0;
     if (ok) {
         tile = film_tile(px, py, fv.tiles_x);
-        pixel = (tile << 6) | ((py & 7u) << 3) | (px & 7u);  // tile-major: below 2^32 (film_cell)
-        cell = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(fv.cell0) + (size_t)pixel * fv.stride);
+        pixel = (tile << 6) | film_local(px, py);  // below 2^32
+        cell = fv.cell(pixel);
         if (SPEC) {
             v0 = to_fixed(contrib, scale);
         } else {
@@ -164,9 +171,9 @@ __device__ __forceinline__ void deposit(const PhotonParams& p, const FilmView& f
     if (AGG == 0) {
         if (!ok) return;
         mark_tile(p, smask, tile);
-        if (cache && cache_take<SPEC>(*cache, p, pixel, bin, v0, v1, v2)) return;
+        if (cache && cache_take<SPEC>(*cache, p, pixel, cell, v0, v1, v2)) return;
         red_u64(cell, v0);
-        if (!SPEC) { red_u64(cell + 1, v1); red_u64(cell + 2, v2); }
+        if (!SPEC) { red_u64(cell + kTilePixels, v1); red_u64(cell + 2 * kTilePixels, v2); }
         return;
     }
     const unsigned mask = __activemask();
@@ -180,7 +187,7 @@ __device__ __forceinline__ void deposit(const PhotonParams& p, const FilmView& f
     }
     mark_tile(p, smask, tile);
     red_u64(cell, v0);
-    if (!SPEC) { red_u64(cell + 1, v1); red_u64(cell + 2, v2); }
+    if (!SPEC) { red_u64(cell + kTilePixels, v1); red_u64(cell + 2 * kTilePixels, v2); }
 }
 
 __device__ __forceinline__ void record_pair(sc_debug_photon* rec, uint32_t pair, f3 o, f3 d) {
@@ -281,6 +288,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -432,12 +440,12 @@ __device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneV
                 const bool ok = ff ? haze_sample<true>(p, o, d, dist, seg, power, px, py, contrib)
                                    : haze_sample<false>(p, o, d, dist, seg, power, px, py, contrib);
                 if (COUNT) { if (ok) ++cnt->splats; continue; }
-                deposit<SPEC, AGG>(p, film_view(p, SPEC ? bin : 0u), smask, ok, px, py, contrib, cx, cy, cz, p.scale);
+                deposit<SPEC, AGG>(p, film_view<SPEC>(p, bin), smask, ok, px, py, contrib, cx, cy, cz, p.scale);
             }
         } else {
             const HazeSeg hz = ff ? haze_setup<true>(p, o, d, seg, power) : haze_setup<false>(p, o, d, seg, power);
             const HazeView hv = haze_view(p);
-            const FilmView fv = film_view(p, SPEC ? bin : 0u);
+            const FilmView fv = film_view<SPEC>(p, bin);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint32_t draw24 = r.u32() >> 8;
@@ -479,7 +487,7 @@ template <bool SPEC, bool G>
 __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& h, Rng& r, float cx, float cy, float cz,
                                           uint32_t bin, uint32_t* smask, CellCacheOf<SPEC>* cache) {
     const HazeView v = haze_view(p);
-    const FilmView fv = film_view(p, SPEC ? bin : 0u);
+    const FilmView fv = film_view<SPEC>(p, bin);
     uint32_t pixel[4];
     float weight[4];  // -1: not in frame
 #pragma unroll
@@ -501,24 +509,23 @@ __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& 
             w *= rr * rr * rr;
         }
         weight[k] = ok ? w : -1.0f;
-        pixel[k] = (film_tile(px, py, fv.tiles_x) << 6) | ((py & 7u) << 3) | (px & 7u);
+        pixel[k] = (film_tile(px, py, fv.tiles_x) << 6) | film_local(px, py);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (weight[k] != -1.0f) {
             mark_tile(p, smask, pixel[k] >> 6);
-            unsigned long long* cell = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(fv.cell0) +
-                                                                             (size_t)pixel[k] * fv.stride);
+            unsigned long long* cell = fv.cell(pixel[k]);
             if (SPEC) {
                 const unsigned long long x = to_fixed(weight[k], 1.0f);
-                if (!cache || !cache_take<SPEC>(*cache, p, pixel[k], bin, x, 0ull, 0ull)) red_u64(cell, x);
+                if (!cache || !cache_take<SPEC>(*cache, p, pixel[k], cell, x, 0ull, 0ull)) red_u64(cell, x);
             } else {
                 const unsigned long long x = to_fixed(cx * weight[k], 1.0f), y = to_fixed(cy * weight[k], 1.0f),
                                          z = to_fixed(cz * weight[k], 1.0f);
-                if (!cache || !cache_take<SPEC>(*cache, p, pixel[k], 0u, x, y, z)) {
+                if (!cache || !cache_take<SPEC>(*cache, p, pixel[k], cell, x, y, z)) {
                     red_u64(cell, x);
-                    red_u64(cell + 1, y);
-                    red_u64(cell + 2, z);
+                    red_u64(cell + kTilePixels, y);
+                    red_u64(cell + 2 * kTilePixels, z);
                 }
             }
         }
@@ -627,7 +634,7 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
                 else haze_four<SPEC, true>(p, hz, r, cx, cy, cz, bin, smask, cache);
             } else {
                 const HazeView hv = haze_view(p);
-                const FilmView fv = film_view(p, SPEC ? bin : 0u);
+                const FilmView fv = film_view<SPEC>(p, bin);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const uint32_t draw24 = r.u32() >> 8;
@@ -635,7 +642,7 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
                     float contrib;
                     const bool ok = ff ? haze_fast<true>(p, hv, hz, draw24, px, py, contrib)
                                        : haze_fast<false>(p, hv, hz, draw24, px, py, contrib);
-                    deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f, cache, bin);
+                    deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f, cache);
                 }
             }
             ++bounce;
