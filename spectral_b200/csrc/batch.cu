@@ -18,7 +18,7 @@ constexpr size_t kCmfBytes16 = (3 * kTableN * sizeof(float) + 15) / 16 * 16;  //
 
 struct alignas(16) WarpSlot {
     PhotonParams p;
-    sc_primitive prims[kBatchPrims];
+    alignas(16) sc_primitive prims[kBatchPrims];
     sc_plane planes[kBatchPlanes];
     sc_material mats[kBatchPrims];
 };

@@ -17,7 +17,7 @@ constexpr uint32_t kBatchMaskWords = 512;
 // What one warp stages for its current job (byte image copied as 16-byte words).
 struct alignas(16) BatchSlotImage {
     PhotonParams p;
-    sc_primitive prims[kBatchPrims];
+    alignas(16) sc_primitive prims[kBatchPrims];
     sc_plane planes[kBatchPlanes];
     sc_material mats[kBatchPrims];
 };

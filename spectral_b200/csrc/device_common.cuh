@@ -123,8 +123,9 @@ __host__ __device__ __forceinline__ float tab_sample(const float* col, float nm)
 // reflectance are in scatter() below) ----
 __device__ __forceinline__ f3 reflect3(f3 d, f3 n) { return sub(d, mul(n, 2.0f * dot(d, n))); }
 // ---- scene in shared memory ------------------------------------------------
+static_assert(sizeof(sc_primitive) == 32 && sizeof(sc_plane) == 16, "records are read 16 bytes at a time");
 struct SceneView {
-    const sc_primitive* prims;
+    const sc_primitive* prims;  // 16-byte aligned, and so are the planes
     const sc_plane* planes;
     const sc_material* mats;
     uint32_t n_prims;
@@ -139,12 +140,11 @@ __device__ __forceinline__ bool below_tmin(float num, float a, float tmin) { ret
 
 // Most rays that meet a sphere again start on it: the root they start from is
 // rejected without its division, and so are both roots of a ray that leaves.
-__device__ __forceinline__ bool sphere_hit(const sc_primitive& pr, f3 o, f3 d, float tmin, float tmax, Hit& h) {
-    f3 c = ld3(pr.center);
+__device__ __forceinline__ bool sphere_hit(f3 c, float radius, f3 o, f3 d, float tmin, float tmax, Hit& h) {
     f3 oc = sub(o, c);
     float a = dot(d, d);
     float half_b = dot(oc, d);
-    float cc = dot(oc, oc) - pr.radius * pr.radius;
+    float cc = dot(oc, oc) - radius * radius;
     float disc = half_b * half_b - a * cc;
     if (disc < 0.0f) return false;
     float sq = sqrtf(disc);
@@ -160,26 +160,34 @@ __device__ __forceinline__ bool sphere_hit(const sc_primitive& pr, f3 o, f3 d, f
         if (t < tmin || t > tmax) return false;
     }
     f3 p = add(o, mul(d, t));
-    f3 outward = vdiv(sub(p, c), pr.radius);
+    f3 outward = vdiv(sub(p, c), radius);
     bool ff = dot(outward, d) < 0.0f;
     h.t = t; h.point = p; h.normal = ff ? outward : neg(outward); h.front_face = ff;
     return true;
 }
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Slabs of a convex solid.  Only two kinds of planes need their division: those
 // the ray enters through from outside (denom < 0, dist > 0) and those it leaves
 // from inside (denom > 0, dist < 0).  An entry plane with the origin inside has
 // t <= 0 < tmin: it is never the hit, and when it exceeds t_exit the solid is
 // missed either way.  An exit plane with the origin outside has t <= 0: the solid
 // is behind the ray.  (Comparisons are written so that NaN takes the division.)
-__device__ __forceinline__ bool solid_hit(const SceneView& S, const sc_primitive& pr, f3 o, f3 d, float tmin, float tmax, Hit& h) {
+__device__ __forceinline__ bool solid_hit(const SceneView& S, uint32_t start, uint32_t count, f3 o, f3 d, float tmin,
+                                          float tmax, Hit& h) {
+    const float4* planes = reinterpret_cast<const float4*>(S.planes);
     float t_enter = -__int_as_float(0x7f800000), t_exit = __int_as_float(0x7f800000);
     uint32_t en = 0xFFFFFFFFu, ex = 0xFFFFFFFFu;  // planes of t_enter and t_exit
-    const uint32_t end = pr.plane_start + pr.plane_count;
-    for (uint32_t i = pr.plane_start; i < end; ++i) {
-        const sc_plane& pl = S.planes[i];
-        f3 n = ld3(pl.normal);
+    const uint32_t end = start + count;
+    for (uint32_t i = start; i < end; ++i) {
+        const float4 pl = planes[i];
+        const f3 n = mk(pl.x, pl.y, pl.z);
         float denom = dot(n, d);
-        float dist = dot(n, o) + pl.d;
+        float dist = dot(n, o) + pl.w;
         if (fabsf(denom) < 1e-8f) {
             if (dist > 0.0f) return false;
             continue;
@@ -200,7 +208,11 @@ __device__ __forceinline__ bool solid_hit(const SceneView& S, const sc_primitive
     else if (t_exit > tmin) { th = t_exit; hp = ex; }
     else return false;
     if (th > tmax) return false;
-    f3 hn = hp != 0xFFFFFFFFu ? ld3(S.planes[hp].normal) : mk(0.f, 0.f, 0.f);
+    f3 hn = mk(0.f, 0.f, 0.f);
+    if (hp != 0xFFFFFFFFu) {
+        const float4 pl = planes[hp];
+        hn = mk(pl.x, pl.y, pl.z);
+    }
     bool ff = dot(hn, d) < 0.0f;
     h.t = th; h.point = add(o, mul(d, th)); h.normal = ff ? hn : neg(hn); h.front_face = ff;
     return true;
@@ -210,11 +222,12 @@ __device__ __forceinline__ bool scene_hit(const SceneView& S, f3 o, f3 d, Hit& b
     bool any = false;
     float closest = __int_as_float(0x7f800000);
     for (uint32_t i = 0; i < S.n_prims; ++i) {
-        const sc_primitive& pr = S.prims[i];
+        const float4 ball = reinterpret_cast<const float4*>(S.prims)[2 * i];
+        const uint4 meta = reinterpret_cast<const uint4*>(S.prims)[2 * i + 1];  // first plane, planes, kind, material
         Hit h;
-        bool ok = pr.kind == 0u ? sphere_hit(pr, o, d, 1e-3f, closest, h)
-                : (pr.kind == 1u ? solid_hit(S, pr, o, d, 1e-3f, closest, h) : false);
-        if (ok) { closest = h.t; best = h; mat = pr.material; any = true; }
+        bool ok = meta.z == 0u ? sphere_hit(mk(ball.x, ball.y, ball.z), ball.w, o, d, 1e-3f, closest, h)
+                : (meta.z == 1u ? solid_hit(S, meta.x, meta.y, o, d, 1e-3f, closest, h) : false);
+        if (ok) { closest = h.t; best = h; mat = meta.w; any = true; }
     }
     return any;
 }
@@ -246,9 +259,17 @@ __device__ __forceinline__ void scatter(const sc_material& m, f3 wo, const Hit& 
     float cos_t = 0.0f;
     if (!(sin_t2 >= 1.0f)) {
         cos_t = sqrtf(1.0f - sin_t2);
-        const float rs = (n1 * c - n2 * cos_t) / (n1 * c + n2 * cos_t);
-        const float rp = (n1 * cos_t - n2 * c) / (n1 * cos_t + n2 * c);
-        mirror = u < 0.5f * (rs * rs + rp * rp);
+        // the reflectance from approximate reciprocals, within 2^-20, decides unless the
+        // draw lies next to it
+        const float sa = n1 * c, sb = n2 * cos_t, pa = n1 * cos_t, pb = n2 * c;
+        float rs = (sa - sb) * rcp_approx(sa + sb), rp = (pa - pb) * rcp_approx(pa + pb);
+        float reflect = 0.5f * __fmaf_rn(rs, rs, rp * rp);
+        if (!(fabsf(u - reflect) > 4e-6f)) {
+            rs = (sa - sb) / (sa + sb);
+            rp = (pa - pb) / (pa + pb);
+            reflect = 0.5f * (rs * rs + rp * rp);
+        }
+        mirror = u < reflect;
     }
     if (mirror) { dir = reflect3(wo, h.normal); return; }
     if (cos_i > 1.0f) cos_t = sqrtf(1.0f - eta * eta * (1.0f - cos_i * cos_i));

@@ -289,12 +289,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return y;
 }
 
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Per-segment constants.  `segs` is seg * 2^-24 for the uniform estimator
 // (t = (draw >> 8) * segs, the same product the reference rounds) and
 // expm1(-sigma_t seg) for free-flight distances.

@@ -41,7 +41,7 @@ constexpr float kLambdaMin = 380.0f, kLambdaRange = 350.0f;
 struct TracerSmem {
     TracerParams p;
     float4 table[kTableN + 1];  // x, y, z and illuminant of a row; the last row twice
-    sc_primitive prims[SC_MAX_PRIMS];
+    alignas(16) sc_primitive prims[SC_MAX_PRIMS];
     sc_material mats[SC_MAX_PRIMS];
     float4 bounds[SC_MAX_PRIMS];
 };
@@ -137,12 +137,13 @@ __device__ __forceinline__ bool scene_hit_bounded(const TracerSmem& s, const Sce
     bool any = false;
     float closest = __int_as_float(0x7f800000);
     for (uint32_t i = 0; i < S.n_prims; ++i) {
-        const sc_primitive& pr = S.prims[i];
-        if (pr.kind == 1u && misses_bound(s.bounds[i], o, d)) continue;
+        const float4 ball = reinterpret_cast<const float4*>(S.prims)[2 * i];
+        const uint4 meta = reinterpret_cast<const uint4*>(S.prims)[2 * i + 1];  // first plane, planes, kind, material
+        if (meta.z == 1u && misses_bound(s.bounds[i], o, d)) continue;
         Hit h;
-        bool ok = pr.kind == 0u ? sphere_hit(pr, o, d, 1e-3f, closest, h)
-                : (pr.kind == 1u ? solid_hit(S, pr, o, d, 1e-3f, closest, h) : false);
-        if (ok) { closest = h.t; best = h; mat = pr.material; any = true; }
+        bool ok = meta.z == 0u ? sphere_hit(mk(ball.x, ball.y, ball.z), ball.w, o, d, 1e-3f, closest, h)
+                : (meta.z == 1u ? solid_hit(S, meta.x, meta.y, o, d, 1e-3f, closest, h) : false);
+        if (ok) { closest = h.t; best = h; mat = meta.w; any = true; }
     }
     return any;
 }
@@ -157,11 +158,8 @@ __device__ __forceinline__ void trace_hit(const TracerSmem& s, const SceneView& 
     uint32_t kind = any ? 1u : 0u;
     t = any ? h.t : __int_as_float(0x7f800000);
     if (s.p.em_radius > 0.0f) {
-        sc_primitive em;
-        em.center[0] = s.p.em_center.x; em.center[1] = s.p.em_center.y; em.center[2] = s.p.em_center.z;
-        em.radius = s.p.em_radius;
         Hit he;
-        if (sphere_hit(em, o, d, 1e-3f, t, he)) { kind = 2u; t = he.t; }
+        if (sphere_hit(s.p.em_center, s.p.em_radius, o, d, 1e-3f, t, he)) { kind = 2u; t = he.t; }
     }
     n = h.normal;
     info = mi | (((any && h.front_face) ? 1u : 0u) << 16) | (kind << 24);
