@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p,
         const uint64_t base = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + warp) * chunk;
         if (base < p.photon_count) {
             const uint32_t b0 = (uint32_t)base;
-            trace_group_range<SPEC, AGG, FF>(
+            trace_group_range<SPEC, AGG, FF, true>(
                 p, S, cmf, min(chunk, p.photon_count - b0),
                 [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); }, smask,
                 reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp], cache);
