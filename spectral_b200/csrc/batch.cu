@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256, MINB) batch_kernel(const BatchJobDev* __r
         SceneView S;
         S.prims = slot.prims; S.planes = slot.planes; S.mats = slot.mats; S.n_prims = slot.p.n_prims;
         const uint32_t first = item.begin;
-        trace_group_range<true, AGG, FF, false>(slot.p, S, cmf, item.count, [first](uint32_t k) { return first + k; },
+        trace_group_range<true, AGG, FF, false, false>(slot.p, S, cmf, item.count, [first](uint32_t k) { return first + k; },
                                          cur_words ? mask : nullptr, park[warp]);
         __syncwarp();
     }

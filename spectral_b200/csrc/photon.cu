@@ -35,9 +35,8 @@ __host__ __device__ __forceinline__ size_t park_offset(const PhotonParams& p, ui
 // 256 threads per CTA; MINB CTAs per SM bound the registers (4: 63 registers,
 // no spills; 5: 48 registers, a few spills, more warps in flight).
 // FF: built with free-flight sampling (estimator 3) as well.  EXACT: haze
-// samples in the CPU crate's operation order (per-photon transport only).
-// CACHE: built with the shared-memory cell cache.  chunk: photons of each warp
-// (not EXACT).  cached: use the cache (CACHE only).
+// samples in the CPU crate's operation order.  CACHE: built with the shared-memory
+// cell cache.  chunk: photons of each warp.  cached: use the cache (CACHE only).
 template <bool SPEC, int AGG, int MINB, bool FF, bool EXACT = false, bool CACHE = false>
 __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words, uint32_t chunk,
                                                            uint32_t cached) {
@@ -45,35 +44,28 @@ __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p,
     const float* cmf;
     uint32_t* smask;
     const SceneView S = load_scene(p, smem, &cmf, &smask, mask_words);
-    if (EXACT) {
-        const uint32_t stride = gridDim.x * blockDim.x;
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.photon_count; i += stride)
-            trace_photon<SPEC, AGG, false, false, FF, true>(p, S, cmf, p.photon_base + (p.order ? p.order[i] : i),
-                                                             smask);
-    } else {
-        CellCacheOf<SPEC>* cache = nullptr;
-        if (CACHE && cached) {
-            cache = reinterpret_cast<CellCacheOf<SPEC>*>(smem + park_offset(p, mask_words) +
-                                                         8 * sizeof(ParkedPhotons<SPEC>));
-            cache->clear();
-            __syncthreads();
-        }
-        // one chunk of the launch's photons per warp; CTAs start in launch order, so
-        // the photons in flight stay close in it (the wavelength-ordered dispatch
-        // relies on that)
-        const uint32_t warp = threadIdx.x >> 5;
-        const uint64_t base = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + warp) * chunk;
-        if (base < p.photon_count) {
-            const uint32_t b0 = (uint32_t)base;
-            trace_group_range<SPEC, AGG, FF, true>(
-                p, S, cmf, min(chunk, p.photon_count - b0),
-                [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); }, smask,
-                reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp], cache);
-        }
-        if (CACHE && cached) {
-            __syncthreads();
-            cache->flush(p.film);
-        }
+    CellCacheOf<SPEC>* cache = nullptr;
+    if (CACHE && cached) {
+        cache = reinterpret_cast<CellCacheOf<SPEC>*>(smem + park_offset(p, mask_words) +
+                                                     8 * sizeof(ParkedPhotons<SPEC>));
+        cache->clear();
+        __syncthreads();
+    }
+    // one chunk of the launch's photons per warp; CTAs start in launch order, so
+    // the photons in flight stay close in it (the wavelength-ordered dispatch
+    // relies on that)
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint64_t base = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + warp) * chunk;
+    if (base < p.photon_count) {
+        const uint32_t b0 = (uint32_t)base;
+        trace_group_range<SPEC, AGG, FF, true, EXACT>(
+            p, S, cmf, min(chunk, p.photon_count - b0),
+            [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); }, smask,
+            reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp], cache);
+    }
+    if (CACHE && cached) {
+        __syncthreads();
+        cache->flush(p.film);
     }
     if (smask) {  // publish this CTA's dirty tiles
         __syncthreads();
@@ -91,7 +83,7 @@ __global__ void __launch_bounds__(256) photon_count_kernel(const PhotonParams p,
     unsigned long long seg = 0, spl = 0, sca = 0, ph = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < p.photon_count; i += gridDim.x * blockDim.x) {
         PhotonCounts c = {0u, 0u, 0u};
-        trace_photon<false, 0, false, true>(p, S, cmf, p.photon_base + i, nullptr, &c);
+        trace_photon<false>(p, S, p.photon_base + i, &c);
         seg += c.segments; spl += c.splats; sca += c.scatters; ++ph;
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -110,7 +102,7 @@ __global__ void __launch_bounds__(256) photon_debug_kernel(const PhotonParams p)
     const float* cmf;
     const SceneView S = load_scene(p, smem, &cmf);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < p.photon_count) trace_photon<false, 0, true>(p, S, cmf, i, nullptr);
+    if (i < p.photon_count) trace_photon<true>(p, S, i);
 }
 
 // Surface rim pass (spectral-gpu/src/shaders/volume.wgsl:668-703 and its CPU
@@ -285,11 +277,14 @@ using PhotonKernelFn = void (*)(const PhotonParams, uint32_t, uint32_t, uint32_t
 
 // `few`: film of few cells per pixel (the kernels built with the cell cache).
 static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool few, bool ff, bool exact = false) {
-    // haze samples in the reference's operation order: per-photon transport,
-    // plain atomics, 4 CTAs per SM
+    // haze samples in the reference's operation order: plain atomics, 4 CTAs per SM
     if (exact) {
-        if (ff) return spec ? photon_kernel<true, 0, 4, true, true> : photon_kernel<false, 0, 4, true, true>;
-        return spec ? photon_kernel<true, 0, 4, false, true> : photon_kernel<false, 0, 4, false, true>;
+        if (ff) {
+            if (!spec) return photon_kernel<false, 0, 4, true, true, true>;
+            return few ? photon_kernel<true, 0, 4, true, true, true> : photon_kernel<true, 0, 4, true, true>;
+        }
+        if (!spec) return photon_kernel<false, 0, 4, false, true, true>;
+        return few ? photon_kernel<true, 0, 4, false, true, true> : photon_kernel<true, 0, 4, false, true>;
     }
     // free-flight launches: plain atomics, 4 CTAs per SM
     if (ff) {
@@ -466,26 +461,21 @@ static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& 
     const bool exact = p.haze_exact != 0u;
     const uint32_t mw = photon_mask_words(p);
     const bool spec = p.channels != 3u || p.bins != 0u, few = few_cells(spec, p.channels);
-    uint32_t chunk = 0, grid;
-    if (exact) {
-        const uint32_t need = (p.photon_count - 1u) / 256u + 1u;
-        grid = need < shape.grid ? need : shape.grid;
-    } else {
-        // 32 photons for each warp while the GPU holds all of them; then about two
-        // chunks for each warp that it holds, 64 to 256 photons: the hardware starts
-        // the next CTA where one has ended.  One CTA per resident slot with its share
-        // of the photons ended unevenly (rainbow, 2^26 photons: 8.3 ms against 6.75,
-        // SMs idle 18 % of it); longer chunks do so again (512: 6.79 ms, 2048: 6.98),
-        // shorter ones pay for each warp's last photons and each CTA's setup (2^26
-        // photons in chunks of 64: 7.35 ms; 2^20 photons, 32 bins: 32 210 us, 64 195,
-        // 128 205, 256 230; 2^16: 32 29 us, 64 33, 128 52).
-        const uint64_t held = shape.grid * 8ull, per = p.photon_count / (2ull * held);
-        chunk = p.photon_count <= 32ull * held ? 32u
-                                               : (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
-        grid = (uint32_t)((p.photon_count - 1u) / (8ull * chunk) + 1u);
-    }
-    const bool cached = !exact && few && shape.aggregate == 0 && cache_pays(p, spec ? p.channels : 1u, chunk);
-    const size_t smem = park_offset(p, mw) + (exact ? 0 : park_bytes(spec, cached));
+    // 32 photons for each warp while the GPU holds all of them; then about two
+    // chunks for each warp that it holds, 64 to 256 photons: the hardware starts
+    // the next CTA where one has ended.  One CTA per resident slot with its share
+    // of the photons ended unevenly (rainbow, 2^26 photons: 8.3 ms against 6.75,
+    // SMs idle 18 % of it); longer chunks do so again (512: 6.79 ms, 2048: 6.98),
+    // shorter ones pay for each warp's last photons and each CTA's setup (2^26
+    // photons in chunks of 64: 7.35 ms; 2^20 photons, 32 bins: 32 210 us, 64 195,
+    // 128 205, 256 230; 2^16: 32 29 us, 64 33, 128 52).
+    const uint64_t held = shape.grid * 8ull, per = p.photon_count / (2ull * held);
+    const uint32_t chunk = p.photon_count <= 32ull * held
+                               ? 32u
+                               : (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
+    const uint32_t grid = (uint32_t)((p.photon_count - 1u) / (8ull * chunk) + 1u);
+    const bool cached = few && (exact || shape.aggregate == 0) && cache_pays(p, spec ? p.channels : 1u, chunk);
+    const size_t smem = park_offset(p, mw) + park_bytes(spec, cached);
     const PhotonKernelFn fn = photon_fn(shape, spec, few, free_flight(p), exact);
     if (smem > 48 * 1024) allow_max_smem(reinterpret_cast<const void*>(fn));
     fn<<<grid, 256, smem, s>>>(p, mw, chunk, cached ? 1u : 0u);

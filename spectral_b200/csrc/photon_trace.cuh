@@ -403,19 +403,16 @@ __device__ __forceinline__ void photon_payload(const PhotonParams& p, const floa
     }
 }
 
-// EXACT: haze samples in the CPU crate's operation order (haze_sample);
-// otherwise the fast haze samples, as the grouped transport runs them.
-template <bool SPEC, int AGG, bool DEBUG, bool COUNT = false, bool FFOK = true, bool EXACT = false>
-__device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneView& S, const float* cmf,
-                                             uint32_t idx, uint32_t* smask, PhotonCounts* cnt = nullptr) {
+// One photon on its own: recorded (DEBUG: its states, no samples) or counted (its
+// samples that land in frame, no film).
+template <bool DEBUG>
+__device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneView& S, uint32_t idx,
+                                             PhotonCounts* cnt = nullptr) {
     Rng r = Rng::make(idx, p.seed);
     const float r1 = r.f32();
     const float r2 = r.f32();
     f3 o = add(add(p.corner, mul(p.bu, r1)), mul(p.bv, r2));
     const float lambda = p.lambda_min + p.lambda_range * r.f32();
-    float cx = 0.f, cy = 0.f, cz = 0.f;
-    uint32_t bin = 0;
-    if (!DEBUG) photon_payload(p, cmf, lambda, cx, cy, cz, bin, SPEC);
     f3 d = p.bdir;
     float power = 1.0f;
     uint32_t n_glass = 0xFFFFFFFFu;
@@ -433,26 +430,13 @@ __device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneV
         uint32_t mi = 0;
         const bool any = scene_hit(S, o, d, h, mi);
         const float seg = any ? h.t : p.max_dist;
-        if (COUNT) ++cnt->segments;
-        const bool ff = FFOK && free_flight(p);
         if (DEBUG) {
             r.state += 4u;  // the segment's 4 distance draws
-        } else if (EXACT) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float u = r.f32();
-                const float dist = ff ? haze_distance<true>(p, u, seg) : haze_distance<false>(p, u, seg);
-                uint32_t px, py;
-                float contrib;
-                const bool ok = ff ? haze_sample<true>(p, o, d, dist, seg, power, px, py, contrib)
-                                   : haze_sample<false>(p, o, d, dist, seg, power, px, py, contrib);
-                if (COUNT) { if (ok) ++cnt->splats; continue; }
-                deposit<SPEC, AGG>(p, film_view<SPEC>(p, bin), smask, ok, px, py, contrib, cx, cy, cz, p.scale);
-            }
         } else {
+            ++cnt->segments;
+            const bool ff = free_flight(p);
             const HazeSeg hz = ff ? haze_setup<true>(p, o, d, seg, power) : haze_setup<false>(p, o, d, seg, power);
             const HazeView hv = haze_view(p);
-            const FilmView fv = film_view<SPEC>(p, bin);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint32_t draw24 = r.u32() >> 8;
@@ -460,8 +444,7 @@ __device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneV
                 float contrib;
                 const bool ok = ff ? haze_fast<true>(p, hv, hz, draw24, px, py, contrib)
                                    : haze_fast<false>(p, hv, hz, draw24, px, py, contrib);
-                if (COUNT) { if (ok) ++cnt->splats; continue; }
-                deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f);
+                if (ok) ++cnt->splats;
             }
         }
         if (!any) break;
@@ -475,7 +458,7 @@ __device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneV
         }
         f3 nd;
         float w;
-        if (COUNT) ++cnt->scatters;
+        if (!DEBUG) ++cnt->scatters;
         scatter(m, d, h, nh, r, nd, w);
         power *= w;
         o = h.point;
@@ -584,9 +567,10 @@ constexpr int kGroupLive = 24;
 // segments; when fewer than kGroupLive lanes are left, the live photons are
 // parked in shared memory and the lanes start the next 32, or take up parked
 // photons once these make a full warp.  The photons, their draws and their
-// samples are those of trace_photon (fast haze samples), so the film is
-// bit-identical to it.
-template <bool SPEC, int AGG, bool FFOK, bool TOGETHER, class Id>
+// samples are those of one photon after the other, so the film is too.
+// EXACT: haze samples in the CPU crate's operation order (haze_sample), otherwise
+// the fast ones.
+template <bool SPEC, int AGG, bool FFOK, bool TOGETHER, bool EXACT, class Id>
 __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const SceneView& S, const float* cmf,
                                                   uint32_t count, Id id, uint32_t* smask, ParkedPhotons<SPEC>& park,
                                                   CellCacheOf<SPEC>* cache = nullptr) {
@@ -663,23 +647,37 @@ __device__ __forceinline__ void trace_group_range(const PhotonParams& p, const S
             uint32_t mi = 0;
             const bool any = scene_hit(S, o, d, h, mi);
             const float seg = any ? h.t : p.max_dist;
-            const HazeSeg hz = ff ? haze_setup<true>(p, o, d, seg, power) : haze_setup<false>(p, o, d, seg, power);
-            if (AGG == 0 && FFOK && ff && !p.zbuf) {
-                haze_four<SPEC, true, FFOK, TOGETHER>(p, hz, r, cx, cy, cz, bin, smask, cache);
-            } else if (AGG == 0 && !ff && !p.zbuf && p.estimator != 1u) {
-                if (p.g == 0.0f) haze_four<SPEC, false, false, TOGETHER>(p, hz, r, cx, cy, cz, bin, smask, cache);
-                else haze_four<SPEC, true, false, TOGETHER>(p, hz, r, cx, cy, cz, bin, smask, cache);
-            } else {
-                const HazeView hv = haze_view(p);
+            if constexpr (EXACT) {
                 const FilmView fv = film_view<SPEC>(p, bin);
-#pragma unroll
+#pragma unroll 1
                 for (int k = 0; k < 4; ++k) {
-                    const uint32_t draw24 = r.u32() >> 8;
+                    const float u = r.f32();
+                    const float dist = ff ? haze_distance<true>(p, u, seg) : haze_distance<false>(p, u, seg);
                     uint32_t px, py;
                     float contrib;
-                    const bool ok = ff ? haze_fast<true>(p, hv, hz, draw24, px, py, contrib)
-                                       : haze_fast<false>(p, hv, hz, draw24, px, py, contrib);
-                    deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f, cache);
+                    const bool ok = ff ? haze_sample<true>(p, o, d, dist, seg, power, px, py, contrib)
+                                       : haze_sample<false>(p, o, d, dist, seg, power, px, py, contrib);
+                    deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, p.scale, cache);
+                }
+            } else {
+                const HazeSeg hz = ff ? haze_setup<true>(p, o, d, seg, power) : haze_setup<false>(p, o, d, seg, power);
+                if (AGG == 0 && FFOK && ff && !p.zbuf) {
+                    haze_four<SPEC, true, FFOK, TOGETHER>(p, hz, r, cx, cy, cz, bin, smask, cache);
+                } else if (AGG == 0 && !ff && !p.zbuf && p.estimator != 1u) {
+                    if (p.g == 0.0f) haze_four<SPEC, false, false, TOGETHER>(p, hz, r, cx, cy, cz, bin, smask, cache);
+                    else haze_four<SPEC, true, false, TOGETHER>(p, hz, r, cx, cy, cz, bin, smask, cache);
+                } else {
+                    const HazeView hv = haze_view(p);
+                    const FilmView fv = film_view<SPEC>(p, bin);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t draw24 = r.u32() >> 8;
+                        uint32_t px, py;
+                        float contrib;
+                        const bool ok = ff ? haze_fast<true>(p, hv, hz, draw24, px, py, contrib)
+                                           : haze_fast<false>(p, hv, hz, draw24, px, py, contrib);
+                        deposit<SPEC, AGG>(p, fv, smask, ok, px, py, contrib, cx, cy, cz, 1.0f, cache);
+                    }
                 }
             }
             ++bounce;
