@@ -425,7 +425,7 @@ int sc_photon_film_create(sc_ctx* ctx, const sc_primitive* prims, uint32_t n_pri
     if ((e = f->flags.alloc(flag_words(width, height))) != cudaSuccess) return fail(e);
     if ((e = f->xyz.alloc(3 * npx)) != cudaSuccess) return fail(e);
     if ((e = f->surface.alloc(3 * npx)) != cudaSuccess) return fail(e);
-    if ((e = f->work.alloc(264)) != cudaSuccess) return fail(e);
+    if ((e = f->work.alloc(kSelectWords)) != cudaSuccess) return fail(e);
     if (n_prims && (e = cudaMemcpyAsync(f->prims.p, prims, n_prims * sizeof(sc_primitive), cudaMemcpyHostToDevice, f->stream)) != cudaSuccess) return fail(e);
     if (n_planes && (e = cudaMemcpyAsync(f->planes.p, planes, n_planes * sizeof(sc_plane), cudaMemcpyHostToDevice, f->stream)) != cudaSuccess) return fail(e);
     if (n_mats && (e = cudaMemcpyAsync(f->mats.p, mats, n_mats * sizeof(sc_material), cudaMemcpyHostToDevice, f->stream)) != cudaSuccess) return fail(e);
@@ -638,7 +638,7 @@ int sc_photon_film_auto_expose_p997(sc_photon_film* f, float* exposure) {
     if (k > n - 1) k = n - 1;
     SC_CUDA(launch_composite_select(f->xyz.p, f->surface.p, n, k, f->work.p, f->stream));
     uint32_t bits = 0;
-    SC_CUDA(cudaMemcpyAsync(&bits, f->work.p + 258, 4, cudaMemcpyDeviceToHost, f->stream));
+    SC_CUDA(cudaMemcpyAsync(&bits, f->work.p + kSelectResult, 4, cudaMemcpyDeviceToHost, f->stream));
     SC_CUDA(cudaStreamSynchronize(f->stream));
     float p;
     std::memcpy(&p, &bits, 4);

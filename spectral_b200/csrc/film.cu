@@ -1,5 +1,6 @@
 // Film kernels: sensor reduction / drain, exposure, tonemap, Gaussian gather,
 // and the synthetic atomic-film splat.
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -267,37 +268,84 @@ __global__ void composite_max_y_kernel(const float* __restrict__ xyz, const floa
 }
 
 // Radix select of the k-th smallest composited luminance (values >= 0, so the
-// IEEE bit patterns order like the floats).  work: [0..255] histogram,
-// [256] prefix, [257] k remaining, [258] result bits.
-__global__ void select_hist_kernel(const float* __restrict__ xyz, const float* __restrict__ surface, uint32_t n,
-                                   uint32_t* work, int shift) {
-    __shared__ uint32_t hist[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0u;
+// IEEE bit patterns order like the floats) in three passes of 11, 11 and 10 bits.
+// The CTA that finishes a pass last picks the digit that holds k, so a pass is one
+// launch.  Lanes that share the first lane's digit (mostly the black pixels') count
+// it once.  At 800x800 a call with its read-back takes 53 us (four passes of 8 bits,
+// with a launch for each pick by one thread: 93).
+// work: [0, 2048) histogram, then the digits found, k among their values, the
+// result's bits, CTAs done; zero at the first pass, the histogram zero after each.
+constexpr uint32_t kSelectBins = 2048, kSelectPrefix = kSelectBins, kSelectK = kSelectBins + 1,
+                   kSelectDone = kSelectBins + 3;
+static_assert(kSelectResult == kSelectBins + 2 && kSelectWords == kSelectBins + 4, "work layout");
+template <int PASS>
+__global__ void __launch_bounds__(256) select_kernel(const float* __restrict__ xyz, const float* __restrict__ surface,
+                                                     uint32_t n, uint32_t k0, uint32_t* work) {
+    constexpr int kShift = PASS == 0 ? 21 : PASS == 1 ? 10 : 0, kBits = PASS == 2 ? 10 : 11;
+    __shared__ uint32_t hist[kSelectBins];
+    __shared__ uint32_t warp_sum[8];
+    __shared__ bool last;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    for (uint32_t i = tid; i < kSelectBins; i += blockDim.x) hist[i] = 0u;
     __syncthreads();
-    const uint32_t prefix = work[256];
-    const uint32_t hi_mask = shift >= 24 ? 0u : (0xFFFFFFFFu << (shift + 8));
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float y = xyz[3u * i + 1u] + (surface ? surface[3u * i + 1u] : 0.0f);
-        y = fmaxf(y, 0.0f);
-        const uint32_t bits = __float_as_uint(y);
-        if ((bits & hi_mask) == (prefix & hi_mask)) atomicAdd(&hist[(bits >> shift) & 255u], 1u);
+    const uint32_t prefix = PASS ? work[kSelectPrefix] : 0u;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const uint32_t i = base + tid;
+        bool counts = i < n;
+        uint32_t digit = 0;
+        if (counts) {
+            const float y = fmaxf(xyz[3u * (size_t)i + 1u] + (surface ? surface[3u * (size_t)i + 1u] : 0.0f), 0.0f);
+            const uint32_t bits = __float_as_uint(y);
+            if (PASS) counts = (bits >> (kShift + kBits)) == (prefix >> (kShift + kBits));
+            digit = (bits >> kShift) & ((1u << kBits) - 1u);
+        }
+        const unsigned any = __ballot_sync(0xffffffffu, counts);
+        if (!any) continue;
+        const int src = __ffs(any) - 1;
+        const uint32_t common = __shfl_sync(0xffffffffu, digit, src);
+        const unsigned same = __ballot_sync(0xffffffffu, counts && digit == common);
+        if ((int)lane == src) atomicAdd(&hist[common], (uint32_t)__popc(same));
+        if (counts && digit != common) atomicAdd(&hist[digit], 1u);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
+    for (uint32_t i = tid; i < kSelectBins; i += blockDim.x)
         if (hist[i]) atomicAdd(&work[i], hist[i]);
-}
-__global__ void select_pick_kernel(uint32_t* work, int shift) {
-    if (threadIdx.x != 0) return;
-    uint32_t k = work[257], acc = 0;
-    uint32_t b = 0;
-    for (; b < 255u; ++b) {
-        if (acc + work[b] > k) break;
-        acc += work[b];
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(&work[kSelectDone], 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr uint32_t kPer = kSelectBins / 256;  // digits of each thread
+    uint32_t c[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; ++j) {
+        c[j] = __ldcg(&work[tid * kPer + j]);
+        work[tid * kPer + j] = 0u;
+        sum += c[j];
     }
-    work[256] |= b << shift;
-    work[257] = k - acc;
-    for (int i = 0; i < 256; ++i) work[i] = 0u;
-    if (shift == 0) work[258] = work[256];
+    uint32_t upto = sum;  // inclusive prefix over the threads
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, upto, o);
+        if ((int)lane >= o) upto += v;
+    }
+    if (lane == 31u) warp_sum[tid >> 5] = upto;
+    __syncthreads();
+    for (uint32_t w = 0; w < (tid >> 5); ++w) upto += warp_sum[w];
+    const uint32_t k = PASS ? work[kSelectK] : k0;
+    uint32_t below = upto - sum;
+    __syncthreads();  // every thread has read k
+    if (below <= k && k < upto) {
+        uint32_t j = 0;
+#pragma unroll
+        for (uint32_t q = 0; q + 1u < kPer; ++q)
+            if (j == q && below + c[q] <= k) { below += c[q]; ++j; }
+        const uint32_t found = prefix | ((tid * kPer + j) << kShift);
+        work[kSelectPrefix] = found;
+        work[kSelectK] = k - below;
+        if (PASS == 2) work[kSelectResult] = found;
+    }
+    if (tid == 0) work[kSelectDone] = 0u;
 }
 
 __global__ void to_rgb8_kernel(const float* __restrict__ xyz, const float* __restrict__ surface, uint32_t n,
@@ -464,17 +512,13 @@ cudaError_t launch_composite_max_y(const float* xyz, const float* surface, uint3
 
 cudaError_t launch_composite_select(const float* xyz, const float* surface, uint32_t n, uint32_t k, uint32_t* work,
                                     cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(work, 0, 259 * sizeof(uint32_t), s);
+    cudaError_t e = cudaMemsetAsync(work, 0, kSelectWords * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    e = cudaMemcpyAsync(work + 257, &k, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return e;
-    uint32_t grid = (n + 255) / 256;
-    if (grid > 1184) grid = 1184;
-    if (grid == 0) grid = 1;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        select_hist_kernel<<<grid, 256, 0, s>>>(xyz, surface, n, work, shift);
-        select_pick_kernel<<<1, 32, 0, s>>>(work, shift);
-    }
+    // two CTAs per SM, at least 1024 pixels each: every CTA adds its digits to one histogram
+    const uint32_t need = (n + 1023u) / 1024u, grid = need < 296u ? std::max(need, 1u) : 296u;
+    select_kernel<0><<<grid, 256, 0, s>>>(xyz, surface, n, k, work);
+    select_kernel<1><<<grid, 256, 0, s>>>(xyz, surface, n, k, work);
+    select_kernel<2><<<grid, 256, 0, s>>>(xyz, surface, n, k, work);
     return cudaGetLastError();
 }
 

@@ -141,8 +141,10 @@ cudaError_t launch_reduce_many(const FilmDesc* descs, uint32_t n_films, uint32_t
 
 cudaError_t launch_composite_max_y(const float* xyz, const float* surface, uint32_t n_pixels,
                                    uint32_t* out_bits, cudaStream_t s);
+// `work`: kSelectWords u32; the value's bits are left in work[kSelectResult].
+constexpr uint32_t kSelectWords = 2052, kSelectResult = 2050;
 cudaError_t launch_composite_select(const float* xyz, const float* surface, uint32_t n_pixels,
-                                    uint32_t k, uint32_t* work /*260 u32*/, cudaStream_t s);
+                                    uint32_t k, uint32_t* work, cudaStream_t s);
 cudaError_t launch_to_rgb8(const float* xyz, const float* surface, uint32_t n_pixels, float exposure,
                            uint8_t* out, cudaStream_t s);
 cudaError_t launch_gather_rgba8(const float* xyz, const float* surface, uint32_t w, uint32_t h,
