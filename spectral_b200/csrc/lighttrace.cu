@@ -158,17 +158,21 @@ __global__ void __launch_bounds__(256) zbuffer_kernel(sc_camera cam, uint32_t w,
     out[(size_t)py * w + px] = t_scene < t_floor ? t_scene : t_floor;
 }
 
-int upload_scene(const sc_primitive* prims, uint32_t np, const sc_plane* planes, uint32_t npl,
+// The calls' device memory comes from the context's pool, on the default stream that
+// they run on: a cudaMalloc and a cudaFree for each buffer of each call, which also
+// wait for the device, took 1.3 of the 2.3 ms of a 512x512 caustic of 2^18 photons.
+int upload_scene(const sc_ctx* ctx, const sc_primitive* prims, uint32_t np, const sc_plane* planes, uint32_t npl,
                  const sc_material* mats, uint32_t nm, DevBuf<sc_primitive>& dp, DevBuf<sc_plane>& dpl,
                  DevBuf<sc_material>& dm) {
     const int rc = check_scene(np, npl, nm, prims, planes, mats);
     if (rc != SC_OK) return rc;
+    dp.bind(ctx->pool, 0); dpl.bind(ctx->pool, 0); dm.bind(ctx->pool, 0);
     SC_CUDA(dp.alloc(np ? np : 1));
     SC_CUDA(dpl.alloc(npl ? npl : 1));
     SC_CUDA(dm.alloc(nm ? nm : 1));
-    if (np) SC_CUDA(cudaMemcpy(dp.p, prims, np * sizeof(sc_primitive), cudaMemcpyHostToDevice));
-    if (npl) SC_CUDA(cudaMemcpy(dpl.p, planes, npl * sizeof(sc_plane), cudaMemcpyHostToDevice));
-    if (nm) SC_CUDA(cudaMemcpy(dm.p, mats, nm * sizeof(sc_material), cudaMemcpyHostToDevice));
+    if (np) SC_CUDA(cudaMemcpyAsync(dp.p, prims, np * sizeof(sc_primitive), cudaMemcpyHostToDevice, 0));
+    if (npl) SC_CUDA(cudaMemcpyAsync(dpl.p, planes, npl * sizeof(sc_plane), cudaMemcpyHostToDevice, 0));
+    if (nm) SC_CUDA(cudaMemcpyAsync(dm.p, mats, nm * sizeof(sc_material), cudaMemcpyHostToDevice, 0));
     return SC_OK;
 }
 
@@ -200,14 +204,15 @@ int sc_lighttrace(sc_ctx* ctx, const sc_primitive* prims, uint32_t n_prims, cons
     DevBuf<sc_primitive> dp;
     DevBuf<sc_plane> dpl;
     DevBuf<sc_material> dm;
-    int rc = upload_scene(prims, n_prims, planes, n_planes, mats, n_mats, dp, dpl, dm);
+    int rc = upload_scene(ctx, prims, n_prims, planes, n_planes, mats, n_mats, dp, dpl, dm);
     if (rc != SC_OK) return rc;
     const size_t n = 3ull * width * height;
     DevBuf<unsigned long long> film;
     DevBuf<float> out;
+    film.bind(ctx->pool, 0); out.bind(ctx->pool, 0);
     SC_CUDA(film.alloc(n));
     SC_CUDA(out.alloc(n));
-    SC_CUDA(cudaMemset(film.p, 0, film.bytes()));
+    SC_CUDA(cudaMemsetAsync(film.p, 0, film.bytes(), 0));
     LightParams p;
     std::memset(&p, 0, sizeof p);
     p.corner = ld3(beam->corner); p.bu = ld3(beam->u); p.bv = ld3(beam->v); p.bdir = ld3(beam->dir);
@@ -245,9 +250,10 @@ int sc_scene_zbuffer(sc_ctx* ctx, const sc_primitive* prims, uint32_t n_prims, c
     DevBuf<sc_primitive> dp;
     DevBuf<sc_plane> dpl;
     DevBuf<sc_material> dm;
-    int rc = upload_scene(prims, n_prims, planes, n_planes, mats, n_mats, dp, dpl, dm);
+    int rc = upload_scene(ctx, prims, n_prims, planes, n_planes, mats, n_mats, dp, dpl, dm);
     if (rc != SC_OK) return rc;
     DevBuf<float> z;
+    z.bind(ctx->pool, 0);
     SC_CUDA(z.alloc((size_t)width * height));
     const size_t smem = n_prims * sizeof(sc_primitive) + n_planes * sizeof(sc_plane) + n_mats * sizeof(sc_material);
     dim3 block(16, 16), grid((width + 15) / 16, (height + 15) / 16);
