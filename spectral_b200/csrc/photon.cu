@@ -11,6 +11,7 @@
 // Splats land in a 64-bit fixed-point film with red.global.add.u64; the film is
 // tile-major (8x8 pixel tiles) and every touched tile raises a dirty flag so the
 // drain/reduce pass reads only tiles that received light.
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -36,7 +37,8 @@ __host__ __device__ __forceinline__ size_t park_offset(const PhotonParams& p, ui
 // no spills; 5: 48 registers, a few spills, more warps in flight).
 // FF: built with free-flight sampling (estimator 3) as well.  EXACT: haze
 // samples in the CPU crate's operation order.  CACHE: built with the shared-memory
-// cell cache.  chunk: photons of each warp.  cached: use the cache (CACHE only).
+// cell cache.  chunk: photons of each warp.  cached: slots of
+// the cache, 0: none (CACHE only).
 template <bool SPEC, int AGG, int MINB, bool FF, bool EXACT = false, bool CACHE = false>
 __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words, uint32_t chunk,
                                                            uint32_t cached) {
@@ -44,10 +46,9 @@ __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p,
     const float* cmf;
     uint32_t* smask;
     const SceneView S = load_scene(p, smem, &cmf, &smask, mask_words);
-    CellCacheOf<SPEC>* cache = nullptr;
-    if (CACHE && cached) {
-        cache = reinterpret_cast<CellCacheOf<SPEC>*>(smem + park_offset(p, mask_words) +
-                                                     8 * sizeof(ParkedPhotons<SPEC>));
+    CellCacheOf<SPEC> cells(smem + park_offset(p, mask_words) + 8 * sizeof(ParkedPhotons<SPEC>), cached);
+    CellCacheOf<SPEC>* cache = CACHE && cached ? &cells : nullptr;
+    if (cache) {
         cache->clear();
         __syncthreads();
     }
@@ -63,7 +64,7 @@ __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p,
             [&](uint32_t k) { return p.photon_base + (p.order ? p.order[b0 + k] : b0 + k); }, smask,
             reinterpret_cast<ParkedPhotons<SPEC>*>(smem + park_offset(p, mask_words))[warp], cache);
     }
-    if (CACHE && cached) {
+    if (cache) {
         __syncthreads();
         cache->flush(p.film);
     }
@@ -301,12 +302,10 @@ static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool few, bool 
     return s.minb >= 5 ? photon_kernel<true, 0, 5, false> : photon_kernel<true, 0, 4, false>;
 }
 static bool few_cells(bool spec, uint32_t channels) { return !spec || channels <= kCacheBins; }
-// Shared memory beyond scene + mask: the parked photons of 8 warps, the cache.
-static size_t park_bytes(bool spec, bool cached) {
-    return 16 + (spec ? 8 * sizeof(ParkedPhotons<true>) + (cached ? sizeof(CellCacheOf<true>) : 0)
-                      : 8 * sizeof(ParkedPhotons<false>) + (cached ? sizeof(CellCacheOf<false>) : 0));
+// Shared memory beyond scene + mask: the parked photons of 8 warps.
+static size_t park_bytes(bool spec) {
+    return 16 + 8 * (spec ? sizeof(ParkedPhotons<true>) : sizeof(ParkedPhotons<false>));
 }
-
 void set_haze_consts(PhotonParams& p) {
     const double pi = 3.14159265358979323846;
     const double g = p.g;
@@ -362,7 +361,7 @@ int occupancy_blocks(const void* fn, int block, size_t smem) {
 
 int photon_occupancy_blocks(const LaunchShape& shape, bool spectral, size_t smem) {
     return occupancy_blocks(reinterpret_cast<const void*>(photon_fn(shape, spectral, !spectral, false)),
-                            (int)shape.block, smem + park_bytes(spectral, false));
+                            (int)shape.block, smem + park_bytes(spectral));
 }
 
 uint32_t photon_mask_words(const PhotonParams& p) {
@@ -372,20 +371,23 @@ uint32_t photon_mask_words(const PhotonParams& p) {
     return words <= kMaxSmemMaskWords ? words : 0u;
 }
 
-// L2 bytes of the current device, read once per device.
-static size_t l2_bytes() {
+// An attribute of the current device, read once per device (0 if unknown).
+static uint32_t device_attribute(cudaDeviceAttr which) {
     static std::mutex mu;
-    static std::map<int, size_t> cache;
+    static std::map<std::pair<int, int>, uint32_t> cache;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
-    auto it = cache.find(dev);
+    const auto key = std::make_pair(dev, (int)which);
+    auto it = cache.find(key);
     if (it != cache.end()) return it->second;
-    int b = 0;
-    cudaDeviceGetAttribute(&b, cudaDevAttrL2CacheSize, dev);
-    cache.emplace(dev, (size_t)(b > 0 ? b : 0));
-    return (size_t)(b > 0 ? b : 0);
+    int v = 0;
+    cudaDeviceGetAttribute(&v, which, dev);
+    cache.emplace(key, (uint32_t)(v > 0 ? v : 0));
+    return (uint32_t)(v > 0 ? v : 0);
 }
+static size_t l2_bytes() { return device_attribute(cudaDevAttrL2CacheSize); }
+static uint32_t sm_count() { return std::max(device_attribute(cudaDevAttrMultiProcessorCount), 1u); }
 
 // Whether a launch takes the wavelength-ordered dispatch: point / isotropic
 // estimators on a spectral film larger than L2 (order 1) or on any spectral
@@ -430,29 +432,53 @@ cudaError_t launch_photons(const PhotonParams& p, const LaunchShape& shape, cuda
     return e != cudaSuccess ? e : f;
 }
 
-// Whether the cell cache pays: the launch is not small (2^14 photons take as long
-// with it as without: clearing and flushing it is 3 us), and the 32 * chunk
-// first-segment samples of a CTA share cells.  These lie along the beam: the
-// frame's height times the beam's width in pixels, seen from the camera at the
-// beam's start.  Measured at 640x360 (width 2 to 3 pixels): XYZ, 2^16 photons
-// 62 -> 39 us (dsotm), 97 -> 56 (prism), 2^20 641 -> 250, 1017 -> 449; 8 bins, 2^20
-// 212 -> 200, 367 -> 236 (4 samples a cell at XYZ 2^20).  The rainbow's beam (205
-// pixels): XYZ 2^20 325 -> 277 us (0.055 samples a cell), 2^18 103 -> 92 and 2 bins
-// 2^20 162 -> 152 (0.028), but 4 bins 2^20 108 -> 146 and XYZ 2^15 24 -> 29 (0.014):
-// the line lies at 0.02.  A z-buffer takes samples away: 0.055 then lose (148 ->
-// 201), 4 still win (prism 995 -> 464).
-static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk) {
-    if (p.photon_count < (1u << 15)) return false;
-    if (8ull * chunk * 4ull * p.max_bounces > kCacheDeposits) return false;  // 8 warps, 4 samples a segment
+// About the pixels that the samples of the first segments share: they lie along the
+// beam, the frame's height times the beam's width in pixels, seen from the camera at
+// the beam's start (negative: behind the camera).
+static float beam_pixels(const PhotonParams& p) {
     const f3 c = sub(add(p.corner, mul(add(p.bu, p.bv), 0.5f)), p.proj.o);
     const float depth = -dot(c, p.proj.w) / length(p.proj.w);
     const f3 across = cross(p.bdir, p.proj.w);  // on screen, square to the beam
     const float l = length(across);
     float width = length(p.bu) + length(p.bv);
     if (l > 1e-3f * length(p.bdir) * length(p.proj.w)) width = (fabsf(dot(p.bu, across)) + fabsf(dot(p.bv, across))) / l;
-    if (!(depth > 0.0f)) return false;
-    const float pixels = (1.0f + width / depth * (float)p.height / p.proj.vh) * (float)p.height;
+    if (!(depth > 0.0f)) return -1.0f;
+    return (1.0f + width / depth * (float)p.height / p.proj.vh) * (float)p.height;
+}
+
+// Whether the cell cache pays: the launch is not small (2^14 photons take as long
+// with it as without: clearing and flushing it is 3 us), and the 32 * chunk
+// first-segment samples of a CTA share cells (beam_pixels).  Measured at 640x360 (2
+// to 3 pixels wide) without and with it: XYZ, 2^16 photons 88 -> 55 us (prism), 2^20
+// 933 -> 385, 2^22 3243 -> 1300; dsotm 800x800, 4M photons 1161 -> 800; 8 bins, 2^20
+// 265 -> 216 (16 bins take 175 without it).  The rainbow's beam (205 pixels): XYZ 2^20
+// 330 -> 278 us (0.055 samples a cell), 2 bins 188 -> 163 (0.028), but 4 bins 108 -> 146
+// and XYZ 2^15 24 -> 29 (0.014): the line lies at 0.02.  A z-buffer takes samples
+// away: 0.055 then lose (148 -> 201), 4 still win (prism 995 -> 464).
+static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk, float pixels) {
+    if (p.photon_count < (1u << 15)) return false;
+    if (8ull * chunk * 4ull * p.max_bounces > kCacheDeposits) return false;  // 8 warps, 4 samples a segment
+    if (!(pixels > 0.0f)) return false;
     return 32.0f * (float)chunk >= (p.zbuf ? 0.4f : 0.02f) * pixels * (float)cells_per_pixel;
+}
+// Slots of the cell cache beside `smem` bytes of a CTA (228 KB per SM, 1 KB of each
+// CTA taken): what lets 4 CTAs share an SM, or for XYZ films 3, where the hot cells
+// (about 2.5 for each pixel of the beam) find a slot then but not among 4 CTAs, and
+// where chunks are long, or the beam is very wide, and they do neither way.  4 against 3 CTAs, 2^20 photons: 1 to 8
+// bins 217 and 249 us, dsotm XYZ 256x256 205 and 242, 800x800 239 and 281; prism 640x360
+// XYZ 415 and 384 (2^22: 1388 and 1296), dsotm 1600x1200 2^22 955 and 900.  Launches of
+// 32 photons a warp clear and flush 2048 at most (2^16 photons: 42 us against 44).
+static uint32_t cache_slots(bool spec, size_t smem, uint32_t chunk, float pixels) {
+    const size_t slot = spec ? CellCacheOf<true>::kSlotBytes : CellCacheOf<false>::kSlotBytes;
+    auto fit = [&](uint32_t ctas) {
+        const size_t room = (228u * 1024u) / ctas - 1024u;
+        return room > smem ? (uint32_t)((room - smem) / slot) : 0u;
+    };
+    uint32_t n = fit(4);
+    const float hot = 2.5f * pixels;
+    if (!spec && hot > (float)n && (hot <= (float)fit(3) || chunk >= 256u || hot > 16.0f * (float)n)) n = fit(3);
+    for (uint32_t ctas = 3; n < 1024u && ctas >= 1u; --ctas) n = fit(ctas);  // a large mask
+    return std::min(n, chunk <= 32u ? 2048u : 8192u);
 }
 
 static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& shape, cudaStream_t s) {
@@ -470,15 +496,24 @@ static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& 
     // photons in chunks of 64: 7.35 ms; 2^20 photons, 32 bins: 32 210 us, 64 195,
     // 128 205, 256 230; 2^16: 32 29 us, 64 33, 128 52).
     const uint64_t held = shape.grid * 8ull, per = p.photon_count / (2ull * held);
-    const uint32_t chunk = p.photon_count <= 32ull * held
-                               ? 32u
-                               : (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
-    const uint32_t grid = (uint32_t)((p.photon_count - 1u) / (8ull * chunk) + 1u);
-    const bool cached = few && (exact || shape.aggregate == 0) && cache_pays(p, spec ? p.channels : 1u, chunk);
-    const size_t smem = park_offset(p, mw) + park_bytes(spec, cached);
+    uint32_t chunk = p.photon_count <= 32ull * held
+                         ? 32u
+                         : (uint32_t)(per < 64u ? 64u : per > 256u ? 256u : (per + 31u) & ~31ull);
+    const float pixels = beam_pixels(p);
+    const bool cached = few && (exact || shape.aggregate == 0) && cache_pays(p, spec ? p.channels : 1u, chunk, pixels);
+    size_t smem = park_offset(p, mw) + park_bytes(spec);
+    const uint32_t slots = cached ? cache_slots(spec, smem, chunk, pixels) : 0u;
+    smem += slots * (size_t)(spec ? CellCacheOf<true>::kSlotBytes : CellCacheOf<false>::kSlotBytes);
     const PhotonKernelFn fn = photon_fn(shape, spec, few, free_flight(p), exact);
     if (smem > 48 * 1024) allow_max_smem(reinterpret_cast<const void*>(fn));
-    fn<<<grid, 256, smem, s>>>(p, mw, chunk, cached ? 1u : 0u);
+    // a launch of less than one and a half rounds of CTAs is spread over one (dsotm
+    // 400x300, 2^18 photons: 107 -> 90 us); with more rounds, chunks that are no multiple
+    // of 32 cost what the even end saves (prism, 2^20 photons: 169 us against 182)
+    const uint64_t resident = (uint64_t)sm_count() * (uint32_t)occupancy_blocks(reinterpret_cast<const void*>(fn), 256, smem);
+    if (chunk > 32u && chunk <= 128u && 2ull * (p.photon_count / (8ull * chunk)) < 3ull * resident)
+        chunk = std::max(32u, (uint32_t)((p.photon_count - 1u) / (8ull * resident) + 1u));
+    const uint32_t grid = (uint32_t)((p.photon_count - 1u) / (8ull * chunk) + 1u);
+    fn<<<grid, 256, smem, s>>>(p, mw, chunk, slots);
     return cudaGetLastError();
 }
 

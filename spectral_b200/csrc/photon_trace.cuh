@@ -93,37 +93,40 @@ __device__ __forceinline__ FilmView film_view(const PhotonParams& p, uint32_t bi
 
 // Shared-memory sums of the film cells a CTA deposits to most often, for films
 // with few cells per pixel: the photons of a narrow beam meet in a few hundred
-// pixels, and every photon of the launch adds to the same cells of each.  L2 adds
-// to one 128-byte line a few times slower than to several (XYZ films took 3 to 5
-// times as long as 32-bin films of the same photons).  A cell (the three of an XYZ
-// pixel, the one of a spectral film's pixel and bin) takes the slot its hash names
-// if that is free; others go straight to the film.  Sums are two 32-bit words per
-// value (12 low bits, and the rest), so that values below 2^23 stay exact over
-// kCacheDeposits deposits; launches whose CTAs could make more do without.
-constexpr uint64_t kCacheDeposits = 1u << 20;
+// pixels, and every photon of the launch adds to the same cells of each.  A cell (the
+// three values of an XYZ pixel, the one of a spectral film's pixel and bin) takes the
+// slot its hash names if that is free; others go straight to the film.  A sum is a
+// 32-bit word per value and a count of its carries (XYZ: 10 bits of one word each):
+// one shared atomic per value, and a second one only where a word wraps.  Values
+// below 2^22 stay exact over kCacheDeposits deposits (2^9 carries); launches whose
+// CTAs could make more do without.  (Two words per value, both added to: 8 bins 237
+// us against 216, dsotm 256x256 XYZ 235 against 205 for 2^20 photons.)
 // V: values per cell.
+constexpr uint64_t kCacheDeposits = 1u << 19;
 template <int V>
 struct CellCache {
-    static constexpr uint32_t kLog2 = V == 3 ? 11u : 12u, kSlots = 1u << kLog2;
-    static constexpr uint32_t kFree = 0xFFFFFFFFu;
-    uint32_t key[kSlots];         // the cell's position in the film (XYZ: its pixel, tile-major), or free
-    uint32_t sum[2 * V][kSlots];  // low and high words of the values
+    static constexpr uint32_t kFree = 0xFFFFFFFFu, kSlotBytes = 4u * (V + 2u);
+    uint32_t slots;
+    uint32_t* key;  // slots: the cell's position in the film (XYZ: its pixel, tile-major), or free
+    uint32_t* sum;  // V x slots: low words of the values
+    uint32_t* carry;
+    __device__ __forceinline__ CellCache(void* at, uint32_t n)
+        : slots(n), key(static_cast<uint32_t*>(at)), sum(key + n), carry(sum + V * n) {}
     __device__ __forceinline__ void clear() {
-        for (uint32_t i = threadIdx.x; i < kSlots; i += blockDim.x) {
-            key[i] = kFree;
-#pragma unroll
-            for (int k = 0; k < 2 * V; ++k) sum[k][i] = 0u;
-        }
+        for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) key[i] = kFree;
+        for (uint32_t i = threadIdx.x; i < (V + 1u) * slots; i += blockDim.x) sum[i] = 0u;  // and the carries
     }
     // Adds the sums to the film.
     __device__ __forceinline__ void flush(unsigned long long* film) const {
-        for (uint32_t i = threadIdx.x; i < kSlots; i += blockDim.x) {
+        for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) {
             if (key[i] == kFree) continue;
             unsigned long long* cell = V == 1 ? film + key[i]
                                               : film + (size_t)(key[i] >> 6) * (V * kTilePixels) + (key[i] & 63u);
 #pragma unroll
-            for (int k = 0; k < V; ++k)
-                red_u64(cell + k * kTilePixels, (unsigned long long)sum[2 * k][i] + ((unsigned long long)sum[2 * k + 1][i] << 12));
+            for (int k = 0; k < V; ++k) {
+                const uint32_t c = V == 1 ? carry[i] : (carry[i] >> (10 * k)) & 1023u;
+                red_u64(cell + k * kTilePixels, (unsigned long long)sum[k * slots + i] | ((unsigned long long)c << 32));
+            }
         }
     }
     // Whether the values went into the cache.
@@ -131,22 +134,24 @@ struct CellCache {
         unsigned long long any = 0;
 #pragma unroll
         for (int c = 0; c < V; ++c) any |= v[c];
-        if (any >> 23) return false;
-        const uint32_t slot = (k * 0x9E3779B1u) >> (32u - kLog2);
+        if (any >> 22) return false;
+        const uint32_t slot = __umulhi(k * 0x9E3779B1u, slots);
         uint32_t t = key[slot];
         if (t == kFree) t = atomicCAS(&key[slot], kFree, k);
         if (t != k && t != kFree) return false;
+        uint32_t wrapped = 0;
 #pragma unroll
         for (int c = 0; c < V; ++c) {
-            atomicAdd(&sum[2 * c][slot], (uint32_t)v[c] & 0xFFFu);
-            atomicAdd(&sum[2 * c + 1][slot], (uint32_t)v[c] >> 12);
+            const uint32_t x = (uint32_t)v[c], old = atomicAdd(&sum[c * slots + slot], x);
+            if (old + x < old) wrapped |= 1u << (10 * c);
         }
+        if (wrapped) atomicAdd(&carry[slot], wrapped);
         return true;
     }
 };
-// Spectral films of up to this many bins may go through the cache (2^20 photons
-// of the narrow prism beam: 1 bin 1053 -> 239 us, 4 bins 387 -> 223, 8 bins
-// 367 -> 236; 16 bins take 218 without it, 32 bins 200).
+// Spectral films of up to this many bins may go through the cache (2^20 photons of
+// the narrow prism beam without and with it: 1 bin 469 -> 216 us, 4 bins 353 -> 219, 8
+// bins 265 -> 216; 16 bins take 175 without it).
 constexpr uint32_t kCacheBins = 8;
 // No cache (a null pointer of it): films of many bins, and small launches.
 template <bool SPEC> using CellCacheOf = CellCache<SPEC ? 1 : 3>;
