@@ -457,7 +457,8 @@ static float beam_pixels(const PhotonParams& p) {
 // away: 0.055 then lose (148 -> 201), 4 still win (prism 995 -> 464).
 static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk, float pixels) {
     if (p.photon_count < (1u << 15)) return false;
-    if (8ull * chunk * 4ull * p.max_bounces > kCacheDeposits) return false;  // 8 warps, 4 samples a segment
+    // 8 warps of at most 256 photons, 4 samples a segment
+    if (8ull * 256ull * 4ull * p.max_bounces > kCacheDeposits) return false;
     if (!(pixels > 0.0f)) return false;
     return 32.0f * (float)chunk >= (p.zbuf ? 0.4f : 0.02f) * pixels * (float)cells_per_pixel;
 }
