@@ -74,9 +74,9 @@ static size_t mask_smem(uint32_t w, uint32_t h) {
 }
 
 // The launch shape of single-film traces: 256-thread CTAs, 4 per SM, the
-// wavelength-ordered dispatch for spectral films larger than L2.  The environment
+// wavelength-ordered dispatch where a launch touches more than L2 holds.  The environment
 // variables SPECTRAL_CUDA_AGGREGATE, SPECTRAL_CUDA_MINB (4 or 5) and
-// SPECTRAL_CUDA_ORDER (0 never, 1 large spectral films, 2 every spectral film)
+// SPECTRAL_CUDA_ORDER (0 never, 1 by that rule, 2 every spectral film)
 // override it for measurements; every setting gives the same film bits.
 static int default_shape(sc_ctx* ctx, bool spectral, int aggregate, size_t smem, LaunchShape& s,
                          uint32_t estimator = 0) {

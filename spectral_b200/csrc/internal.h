@@ -31,7 +31,7 @@ struct alignas(16) PhotonParams {
     const float* cmf;                 // device 3x71 (xbar, ybar, zbar)
     sc_debug_photon* debug;           // debug launches only
     const uint32_t* order;            // nullable: photon i of the launch is photon_base + order[i]
-    uint32_t haze_exact;              // 1: haze samples in the CPU crate's operation order (per-photon kernel)
+    uint32_t haze_exact;              // 1: haze samples in the CPU crate's operation order
     // Launch constants of the fast haze samples, filled by set_haze_consts()
     // from the fields above just before a launch.
     float hz_sx, hz_sy;               // W / |horizontal|, -H / |vertical|
@@ -45,7 +45,7 @@ void set_haze_consts(PhotonParams& p);
 // Photon launch: CTAs of 256 threads, `grid` CTAs resident on the GPU at once
 // (the unit the photons are divided by), warp aggregation on/off, register
 // bound (minimum CTAs per SM: 4 or 5), and the wavelength-ordered dispatch (0
-// never, 1 for spectral films larger than L2, 2 for every spectral film; its
+// never, 1 where a launch touches more of its film than L2 holds, 2 for every spectral film; its
 // scratch comes from `pool`, and without a pool it is off).
 struct LaunchShape {
     uint32_t block, grid;

@@ -389,17 +389,38 @@ static uint32_t device_attribute(cudaDeviceAttr which) {
 static size_t l2_bytes() { return device_attribute(cudaDevAttrL2CacheSize); }
 static uint32_t sm_count() { return std::max(device_attribute(cudaDevAttrMultiProcessorCount), 1u); }
 
+// About the pixels that the samples of the first segments share: they lie along the
+// beam, the frame's height times the beam's width in pixels, seen from the camera at
+// the beam's start (negative: behind the camera).
+static float beam_pixels(const PhotonParams& p) {
+    const f3 c = sub(add(p.corner, mul(add(p.bu, p.bv), 0.5f)), p.proj.o);
+    const float depth = -dot(c, p.proj.w) / length(p.proj.w);
+    const f3 across = cross(p.bdir, p.proj.w);  // on screen, square to the beam
+    const float l = length(across);
+    float width = length(p.bu) + length(p.bv);
+    if (l > 1e-3f * length(p.bdir) * length(p.proj.w)) width = (fabsf(dot(p.bu, across)) + fabsf(dot(p.bv, across))) / l;
+    if (!(depth > 0.0f)) return -1.0f;
+    return (1.0f + width / depth * (float)p.height / p.proj.vh) * (float)p.height;
+}
+
 // Whether a launch takes the wavelength-ordered dispatch: point / isotropic
-// estimators on a spectral film larger than L2 (order 1) or on any spectral
-// film (order 2), at least 2^16 photons to amortise the sort, and a memory
-// pool for its scratch.
+// estimators on a spectral film, at least 2^16 photons to amortise the sort, a
+// memory pool for its scratch, and (order 1; order 2 orders every such launch) more of
+// the film touched than L2 holds: a film larger than L2, a beam whose own pixels
+// (beam_pixels) have more bytes of bins than L2, and at least two L2s of sectors hit
+// (about 10 samples a photon, 32 bytes each).  Photons in the order of their bins
+// add to the same lines at the same time, so where L2 holds what they touch the order
+// costs.  Not ordered against ordered: rainbow 1920x1080x64 (342 MB under the beam) 2^19
+// photons 426 and 437 us, 2^20 523 and 520, 2^22 941 and 818, 2^26 8.2 and 6.6 ms; prism
+// 1024x1024x32 (2 MB) 2^20 190 and 218 us, 2^24 2.07 and 3.64 ms; dsotm 1600x1200x32 2^24
+// 1.88 and 2.03 ms; 300,000 free-flight photons at 1001x563x31 88 and 114 us.
 static bool ordered_dispatch(const PhotonParams& p, const LaunchShape& shape) {
     if (shape.order == 0 || !shape.pool || p.bins == 0u || p.channels != p.bins || p.order ||
         p.photon_count < (1u << 16))
         return false;
     if (shape.order >= 2) return true;
-    const size_t film = (size_t)p.tiles_x * ((p.height + 7u) / 8u) * kTilePixels * p.channels * 8u;
-    return film > l2_bytes();
+    const size_t film = (size_t)p.tiles_x * ((p.height + 7u) / 8u) * kTilePixels * p.channels * 8u, l2 = l2_bytes();
+    return film > l2 && (double)beam_pixels(p) * p.channels * 8.0 > (double)l2 && p.photon_count * 320ull >= 2ull * l2;
 }
 
 static cudaError_t launch_photons_in(const PhotonParams& p, const LaunchShape& shape, cudaStream_t s);
@@ -430,20 +451,6 @@ cudaError_t launch_photons(const PhotonParams& p, const LaunchShape& shape, cuda
     }
     const cudaError_t f = cudaFreeAsync(buf, s);
     return e != cudaSuccess ? e : f;
-}
-
-// About the pixels that the samples of the first segments share: they lie along the
-// beam, the frame's height times the beam's width in pixels, seen from the camera at
-// the beam's start (negative: behind the camera).
-static float beam_pixels(const PhotonParams& p) {
-    const f3 c = sub(add(p.corner, mul(add(p.bu, p.bv), 0.5f)), p.proj.o);
-    const float depth = -dot(c, p.proj.w) / length(p.proj.w);
-    const f3 across = cross(p.bdir, p.proj.w);  // on screen, square to the beam
-    const float l = length(across);
-    float width = length(p.bu) + length(p.bv);
-    if (l > 1e-3f * length(p.bdir) * length(p.proj.w)) width = (fabsf(dot(p.bu, across)) + fabsf(dot(p.bv, across))) / l;
-    if (!(depth > 0.0f)) return -1.0f;
-    return (1.0f + width / depth * (float)p.height / p.proj.vh) * (float)p.height;
 }
 
 // Whether the cell cache pays: the launch is not small (2^14 photons take as long
