@@ -85,11 +85,11 @@ NCU_TRAFFIC = {
 # active per instruction: the instruction-issue roofline of kernels whose films
 # stay in L2.
 NCU_INST = {
-    "batch": (12734972130 / 2 / 48957886, 21.77, "batch_kernel<0, 4, 0, 0>: two launches on the first 64 scenes "
-                                                  "(48,957,886 photons each), per photon"),
-    "prism": (324289908 / 2 / (1 << 20), 25.60, "photon_kernel: two launches of 2^20 photons, per photon"),
-    "rainbow": (5568513387 / (1 << 26), 23.90, "photon_kernel: one launch of 2^26 photons, per photon"),
-    "tracer": (3642531467 / 58982400, 27.66, "tr_shade, tr_tail, tr_accumulate: the 60 launches of one "
+    "batch": (9731331222 / 2 / 48957886, 26.57, "batch_kernel<0, 4, 0>: two launches on the first 64 scenes "
+                                                 "(48,957,886 photons each), per photon"),
+    "prism": (274675052 / 2 / (1 << 20), 24.67, "photon_kernel: two launches of 2^20 photons, per photon"),
+    "rainbow": (4785072070 / (1 << 26), 23.91, "photon_kernel: one launch of 2^26 photons, per photon"),
+    "tracer": (2577983977 / 58982400, 25.44, "tr_shade, tr_tail, tr_accumulate: the 59 launches of one "
                                              "accumulate(64), per path sample"),
 }
 
