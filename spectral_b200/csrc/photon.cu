@@ -296,7 +296,7 @@ static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool few, bool 
         if (s.minb >= 5) return spec ? photon_kernel<true, 1, 5, false> : photon_kernel<false, 1, 5, false>;
         return spec ? photon_kernel<true, 1, 4, false> : photon_kernel<false, 1, 4, false>;
     }
-    if (few) {  // the cache's shared memory holds 3 CTAs per SM
+    if (few) {  // with the cache, 4 or 3 CTAs per SM (cache_slots)
         return spec ? photon_kernel<true, 0, 4, false, false, true> : photon_kernel<false, 0, 4, false, false, true>;
     }
     return s.minb >= 5 ? photon_kernel<true, 0, 5, false> : photon_kernel<true, 0, 4, false>;
@@ -501,8 +501,7 @@ static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& 
     // of the photons ended unevenly (rainbow, 2^26 photons: 8.3 ms against 6.75,
     // SMs idle 18 % of it); longer chunks do so again (512: 6.79 ms, 2048: 6.98),
     // shorter ones pay for each warp's last photons and each CTA's setup (2^26
-    // photons in chunks of 64: 7.35 ms; 2^20 photons, 32 bins: 32 210 us, 64 195,
-    // 128 205, 256 230; 2^16: 32 29 us, 64 33, 128 52).
+    // photons in chunks of 64: 7.35 ms; 2^20 photons, 64 bins: 64 187 us, 128 169).
     const uint64_t held = shape.grid * 8ull, per = p.photon_count / (2ull * held);
     uint32_t chunk = p.photon_count <= 32ull * held
                          ? 32u
