@@ -478,7 +478,9 @@ __device__ __forceinline__ void trace_photon(const PhotonParams& p, const SceneV
 // branch, so that their chains of approximations overlap: batch pass 22.3 -> 20.5 ms
 // against sample by sample.  (Not with a z-buffer: a sample that is occluded ends
 // there.)  Nearly every deposit is below 2^23 quanta and takes the short rounding:
-// prism, 2^20 photons 174.5 -> 169.5 us, batch pass 19.3 -> 18.9 ms.
+// prism, 2^20 photons 174.5 -> 169.5 us, batch pass 19.3 -> 18.9 ms.  It holds for
+// weights that are not negative, as to_fixed() clamps them: a segment's constant
+// weight carries their sign (sigma_s, 1 - g^2, a reflectance or a length below zero).
 // TOGETHER: the four tiles are tested together (they are lit but for a launch's first
 // photons): 300,000 free-flight photons 114.4 -> 112.0 us, rainbow 6.66 -> 6.59 ms; the
 // batch kernel, which keeps its parameters in shared memory, has no registers for it
@@ -489,6 +491,7 @@ __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& 
                                           uint32_t bin, uint32_t* smask, CellCacheOf<SPEC>* cache) {
     const HazeView v = haze_view(p);
     const FilmView fv = film_view<SPEC>(p, bin);
+    const float hk = SPEC ? fmaxf(h.k, 0.0f) : h.k;  // NaN: 0, as to_fixed() has it
     uint32_t pixel[4];
     float weight[4];  // -1: not in frame
 #pragma unroll
@@ -507,7 +510,7 @@ __device__ __forceinline__ void haze_four(const PhotonParams& p, const HazeSeg& 
         const float dd2 = fmaxf(__fmaf_rn(q, q, h.h2), 1e-6f);
         const float rd = rsqrt_approx(dd2);
         const float dd = dd2 * rd;
-        float w = h.k * ex2_approx(v.kexp * (FF ? dd - t : dd)) * (rd * rd);
+        float w = hk * ex2_approx(v.kexp * (FF ? dd - t : dd)) * (rd * rd);
         if (G) {
             const float den = fmaxf(__fmaf_rn(p.hz_m2g, -(h.s1 * q) * rd, p.hz_g2), 1e-6f);
             const float rr = rsqrt_approx(den);
