@@ -60,9 +60,13 @@ struct alignas(16) StepRec {
 };
 static_assert(sizeof(StepRec) == 64, "step record layout");
 // How a step is splatted (the setup's verdict, kept by its lane): not in frame;
-// by the 8x8 or the 16x16 window; on its own (a larger box, a deposit of 2^23
-// quanta or more, or an empty tent).
+// by the 8x8 or the 16x16 window; on its own (a larger box, one at kWindowEnd, a deposit
+// of 2^23 quanta or more, or an empty tent).
 enum : uint32_t { kStepNone = 0u, kStepWin8 = 1u, kStepWin16 = 2u, kStepAlone = 3u };
+// Boxes of the windows' steps start below this column and row, so two of them differ by
+// less than 2^16 - 16 and window_march can compare their corners modulo 2^16 (only a
+// film of more than 65,520 pixels on a side has others; they go on their own).
+constexpr int kWindowEnd = 65536 - 16;
 constexpr uint32_t kBeamSegs = 64;
 struct alignas(16) BeamWarpSmem {
     BeamSeg seg[kBeamSegs];
@@ -274,7 +278,7 @@ __device__ __forceinline__ uint32_t beam_step(const PhotonParams& p, uint32_t* s
     // where this holds (and the colours are not negative or NaN)
     const bool small = lit && c0 >= 0.0f && c1 >= 0.0f && c2 >= 0.0f &&
                        fmaxf(c0, fmaxf(c1, c2)) * inv < 8388000.0f;
-    const uint32_t side = max(bw, bh);
+    const uint32_t side = x0 < kWindowEnd && y0 < kWindowEnd ? max(bw, bh) : 17u;
     return small && side <= 8u ? kStepWin8 : (small && side <= 16u ? kStepWin16 : kStepAlone);
 }
 
@@ -348,7 +352,8 @@ __device__ __forceinline__ void window_march(const PhotonParams& p, const BeamWa
         const ulonglong2 q0 = rec[0], q1 = rec[1], q2 = rec[2], q3 = rec[3];
         const uint32_t xy = (uint32_t)(q0.x >> 32), nbin = (uint32_t)q3.y, box = (uint32_t)(q3.y >> 32);
         // the box lies in the window where both halves of xy - wxy are within
-        // [0, N - side]: neither they nor the slack left have a sign bit
+        // [0, N - side]: neither they nor the slack left have a sign bit (corners
+        // differ by less than 2^16 - N: kWindowEnd)
         const uint32_t at = xy - wxy, slack = (uint32_t)(N | (N << 16)) - box - at;
         if (((at | slack) & 0x80008000u) || !open || (SPEC && nbin != bin)) {
             const uint32_t x0 = xy & 0xFFFFu, y0 = xy >> 16, bw = box & 0xFFFFu, bh = box >> 16;

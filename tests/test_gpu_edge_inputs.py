@@ -1,10 +1,9 @@
 """Calls at the edges of what the entry points accept: weights below zero, rays
 without a direction, films so wide that 16-bit differences of their columns wrap,
-films of more than 2^32 cells, films of three bins, calls larger than the memory a
+films of more than 2^32 cells or of three bins, calls that take more memory than a
 context keeps.
 
-Films are sums of exact integers, so the comparisons are of every cell."""
-
+Films are sums of exact integers: every cell is compared."""
 import numpy as np
 import pytest
 
@@ -61,3 +60,37 @@ def test_weights_of_both_signs(ctx, monkeypatch):
         raws.append(f.read_raw())
         f.close()
     assert raws[0].sum() > 0 and np.array_equal(raws[0], raws[1])
+
+
+@pytest.mark.parametrize("across", [True, False])
+@pytest.mark.parametrize("bins", [0, 1])
+def test_beam_film_whose_columns_differ_by_almost_2_to_16(ctx, across, bins):
+    """Beams along a film of 65,535 columns (or rows).  Behind a thin slab every
+    photon marches the frame from edge to edge: the last step of one lies on the
+    last column, the first of the next on the first.  In the whole launch a warp has
+    several photons, in the small ones a single photon."""
+    side, thin, n, part = 65_535, 16, 60_000, 3_000
+    w, h = (side, thin) if across else (thin, side)
+    half, far = 700.0, 1000.0  # half the frame's long side, the camera's distance
+    ds = 2.0 * half / 4090.0   # 4096 steps a segment: 4091 from edge to edge, 5 behind it
+    vfov = 2.0 * np.degrees(np.arctan((half * thin / side if across else half) / far))
+    cam = sb.Camera.look_at((0.0, 0.0, far), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), float(vfov), w / h)
+    lo, hi = -half - 0.5 * ds - 0.05, -half - 0.495 * ds
+    scene = sb.Scene(background=0.0)
+    # they start within 0.1 units of the slab, 1 to 9 steps before it, and march
+    # towards the last column, or the last row (downwards)
+    if across:
+        scene.add_solid([((1.0, 0.0, 0.0), -hi), ((-1.0, 0.0, 0.0), lo)], sb.Dielectric(sb.BK7))
+        beam = sb.Beam((lo - 0.11, -0.02, 0.0), (0.1, 0.0, 0.0), (0.0, 0.04, 0.0), (1.0, 0.0, 0.0))
+    else:
+        scene.add_solid([((0.0, 1.0, 0.0), lo), ((0.0, -1.0, 0.0), -hi)], sb.Dielectric(sb.BK7))
+        beam = sb.Beam((-0.02, 0.11 - lo, 0.0), (0.0, -0.1, 0.0), (0.04, 0.0, 0.0), (0.0, -1.0, 0.0))
+    f = sb.GpuPhotonFilm(ctx, scene, cam, beam, w, h, n, 7, 4096.0 * ds * 0.99999, sb.VolWeights(0.5, 0.0, 0.0),
+                         estimator=sb.BEAM, bins=bins, scale_log2=44)
+    f.dispatch_photons(0, n, 7)
+    whole = f.read_raw()
+    f.clear_film()
+    for a in range(0, n, part):
+        f.dispatch_photons(a, a + part, 7)
+    assert whole.sum() > 0 and np.array_equal(f.read_raw(), whole)
+    f.close()
