@@ -336,7 +336,8 @@ __host__ __device__ __forceinline__ uint32_t film_local_pixel(uint32_t at) {
     const uint32_t y = (at >> 1) & 7u;
     return (y << 3) | ((at & 1u) << 2) | (((at >> 4) - y) & 3u);
 }
-// Films have at most 2^28 pixels (beam films 65535 x 65535): below 2^26 tiles.
+// Films have at most 2^28 pixels: about 2^25 tiles (one pixel high or wide), so a tile
+// and a position in it (tile << 6 | film_local) fit 32 bits; a cell's index does not.
 __host__ __device__ __forceinline__ size_t film_cell(uint32_t px, uint32_t py, uint32_t tiles_x, uint32_t channels,
                                                      uint32_t channel = 0) {
     return (size_t)film_tile(px, py, tiles_x) * (kTilePixels * channels) + channel * kTilePixels + film_local(px, py);

@@ -464,6 +464,10 @@ cudaError_t launch_photons(const PhotonParams& p, const LaunchShape& shape, cuda
 // away: 0.055 then lose (148 -> 201), 4 still win (prism 995 -> 464).
 static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk, float pixels) {
     if (p.photon_count < (1u << 15)) return false;
+    // keys are 32-bit cell indices below CellCache::kFree; films of one to seven rows
+    // or columns have up to eight times their pixels in padded cells
+    const uint64_t tiles = (uint64_t)p.tiles_x * ((p.height + 7u) / 8u);
+    if (tiles * kTilePixels * cells_per_pixel > 0xFFFFFFFFull) return false;
     // 8 warps of at most 256 photons, 4 samples a segment
     if (8ull * 256ull * 4ull * p.max_bounces > kCacheDeposits) return false;
     if (!(pixels > 0.0f)) return false;

@@ -160,7 +160,7 @@ template <bool SPEC>
 __device__ __forceinline__ bool cache_take(CellCacheOf<SPEC>& cache, const PhotonParams& p, uint32_t pixel,
                                            const unsigned long long* cell, unsigned long long v0,
                                            unsigned long long v1, unsigned long long v2) {
-    if constexpr (SPEC) return cache.add((uint32_t)(cell - p.film), {v0});  // below 2^31: kCacheBins
+    if constexpr (SPEC) return cache.add((uint32_t)(cell - p.film), {v0});  // below 2^32 - 1: cache_pays()
     else return cache.add(pixel, {v0, v1, v2});
 }
 

@@ -4,13 +4,15 @@ films of more than 2^32 cells or of three bins, calls that take more memory than
 context keeps.
 
 Films are sums of exact integers: every cell is compared."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import spectral_b200 as sb
-from spectral_b200 import specs
+from spectral_b200 import _lib, specs
 from spectral_b200.batch import Batch, prism_jobs
-from helpers import axis_box
+from helpers import axis_box, device_desc
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +96,35 @@ def test_beam_film_whose_columns_differ_by_almost_2_to_16(ctx, across, bins):
         f.dispatch_photons(a, a + part, 7)
     assert whole.sum() > 0 and np.array_equal(f.read_raw(), whole)
     f.close()
+
+
+def test_cell_cache_of_a_film_of_more_than_2_to_32_cells(ctx):
+    """A film one pixel high has eight times its pixels in padded cells: 83,886,080
+    x 1 of 8 bins are 5 * 2^30 cells (43 GB).  A launch that is large enough for the
+    cell cache gives the image of small launches that do without."""
+    import torch
+    w, n = 5 << 24, 60_000
+    scene = sb.Scene(background=0.0)
+    beam = sb.Beam((-3.0, -0.01, 0.0), (0.0, 0.02, 0.0), (0.0, 0.0, 0.02), (1.0, 0.0, 0.0))
+    cam = sb.Camera.look_at((0.0, 0.0, 6.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 30.0, 1.0)
+    keep, images = [], []
+    desc = device_desc(sb, _lib, torch, scene, cam, beam, w, 1, 3, 8, keep, scale_log2=24)  # below 2^22 quanta
+    film = torch.zeros(_lib.lib.sc_film_bytes(w, 1, 8) // 8, dtype=torch.int64, device="cuda")
+    flags = torch.zeros(_lib.lib.sc_film_flag_bytes(w, 1) // 4, dtype=torch.int32, device="cuda")
+    assert film.numel() > 1 << 32
+    for step in (n, 20_000):  # the cache is taken from 2^15 photons on
+        xyz = torch.empty(3 * w, dtype=torch.float32, device="cuda")
+        for a in range(0, n, step):
+            _lib.check(_lib.lib.sc_trace_photons_device(ctx.h, C.byref(desc), a, min(step, n - a),
+                                                        C.c_void_p(film.data_ptr()), C.c_void_p(flags.data_ptr()),
+                                                        None))
+        _lib.check(_lib.lib.sc_sensor_reduce_device(ctx.h, w, 1, 8, 380.0, 730.0, 24, C.c_void_p(film.data_ptr()),
+                                                    C.c_void_p(flags.data_ptr()), C.c_void_p(xyz.data_ptr()), 1,
+                                                    None))
+        torch.cuda.synchronize()
+        images.append(xyz)
+    same = torch.equal(images[0], images[1])
+    beyond = images[1][3 << 26:].sum().item()  # cells from 2^32 on
+    del film, images, xyz
+    torch.cuda.empty_cache()
+    assert same and beyond > 0
