@@ -176,7 +176,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // from inside (denom > 0, dist < 0).  An entry plane with the origin inside has
 // t <= 0 < tmin: it is never the hit, and when it exceeds t_exit the solid is
 // missed either way.  An exit plane with the origin outside has t <= 0: the solid
-// is behind the ray.  (Comparisons are written so that NaN takes the division.)
+// is behind the ray.  (A NaN dist takes the division.)
 __device__ __forceinline__ bool solid_hit(const SceneView& S, uint32_t start, uint32_t count, f3 o, f3 d, float tmin,
                                           float tmax, Hit& h) {
     const float4* planes = reinterpret_cast<const float4*>(S.planes);
@@ -188,8 +188,8 @@ __device__ __forceinline__ bool solid_hit(const SceneView& S, uint32_t start, ui
         const f3 n = mk(pl.x, pl.y, pl.z);
         float denom = dot(n, d);
         float dist = dot(n, o) + pl.w;
-        if (fabsf(denom) < 1e-8f) {
-            if (dist > 0.0f) return false;
+        if (!(fabsf(denom) >= 1e-8f)) {  // parallel to the plane; or NaN, whose quotient moves neither t
+            if (dist > 0.0f && denom == denom) return false;
             continue;
         }
         if (denom < 0.0f) {

@@ -9,10 +9,11 @@ import ctypes as C
 import numpy as np
 import pytest
 
+import oracle
 import spectral_b200 as sb
 from spectral_b200 import _lib, specs
 from spectral_b200.batch import Batch, prism_jobs
-from helpers import axis_box, device_desc
+from helpers import axis_box, device_desc, obeam, oscene
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +129,18 @@ def test_cell_cache_of_a_film_of_more_than_2_to_32_cells(ctx):
     del film, images, xyz
     torch.cuda.empty_cache()
     assert same and beyond > 0
+
+
+@pytest.mark.parametrize("direction", [(float("nan"), 0.0, 0.0), (0.0, 0.0, float("nan"))])
+def test_rays_without_a_direction(ctx, direction):
+    """A NaN direction passes every plane test of a solid by, whichever side of
+    the planes the ray starts on: paths end where the CPU crate's do."""
+    scene = sb.Scene(background=0.0)
+    scene.add_solid(axis_box((-1.0, -1.0, -1.0), (1.0, 1.0, 1.0)), sb.Dielectric(sb.SF11))
+    beam = sb.Beam((-3.0, -0.5, -0.5), (0.0, 0.0, 1.0), (0.0, 1.0, 0.0), direction)
+    cam = sb.Camera.look_at((0.0, 0.0, 8.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 40.0, 1.0)
+    f = sb.GpuPhotonFilm(ctx, scene, cam, beam, 32, 32, 64, 9, 9.0, max_bounces=5)
+    num, _, _ = f.trace_debug(64, 9, 64)
+    p = oracle.vol_params(32, 32, 9, max_dist=9.0, max_bounces=5)
+    assert num.tolist() == [oracle.simulate_photon(oscene(scene), obeam(beam), p, i)[0] for i in range(64)]
+    f.close()
