@@ -311,7 +311,10 @@ int sc_trace_photons_device(sc_ctx* ctx, const sc_trace_desc* desc, uint32_t pho
 int sc_trace_stats_device(sc_ctx* ctx, const sc_trace_desc* desc, uint32_t photon_base, uint32_t count,
                           uint64_t* out_dev, void* stream);
 /* Sensor reduction of a device film to interleaved f32 XYZ (3*w*h, device);
- * drain != 0 also zeroes the film and its tile flags (ready for the next pass). */
+ * drain != 0 also zeroes the film and its tile flags (ready for the next pass).
+ * 3 channels are an XYZ film, here and in sc_sensor_reduce_peers: a spectral film
+ * of exactly 3 bins is reduced by the film object, a batch, the server or
+ * sc_trace_xyz_noalloc, which know its bins. */
 int sc_sensor_reduce_device(sc_ctx* ctx, uint32_t width, uint32_t height, uint32_t channels,
                             float lambda_min, float lambda_max, uint32_t scale_log2,
                             void* film_dev, uint32_t* flags_dev, float* xyz_dev, int drain,

@@ -16,7 +16,7 @@ constexpr int kReduceThreads = 256;
 
 // One film tile (64 pixels x C channels of int64) is staged into shared memory
 // with 16-byte coalesced loads, optionally zeroed behind the load (drain), then
-// reduced per pixel: XYZ film -> value / 2^scale; spectral film -> sum over bins
+// reduced per pixel: XYZ film (no bin weights) -> value / 2^scale; spectral film -> sum over bins
 // of count * bin-averaged CMF (f64 accumulation, fixed order per pixel).
 // Tiles whose dirty flag is clear are never read: their pixels are written as 0.
 //
@@ -83,7 +83,7 @@ __device__ __forceinline__ void reduce_staged(const TileRef& t, bool drain, cons
     const uint32_t C = p.channels, tile = t.tile;
     const uint32_t tx = tile % p.tiles_x, ty = tile / p.tiles_x;
     const uint32_t tid = threadIdx.x;
-    if (!t.dirty || C == 3u) {
+    if (!t.dirty || p.binw == nullptr) {  // clean, or an XYZ film (one of three bins has weights)
         for (uint32_t i = tid; i < kTilePixels * 3u; i += blockDim.x) {
             const uint32_t l = i / 3u, c = i % 3u;
             const uint32_t px = tx * 8u + (l & 7u), py = ty * 8u + (l >> 3);

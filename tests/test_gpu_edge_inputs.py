@@ -13,7 +13,7 @@ import oracle
 import spectral_b200 as sb
 from spectral_b200 import _lib, specs
 from spectral_b200.batch import Batch, prism_jobs
-from helpers import axis_box, device_desc, obeam, oscene
+from helpers import axis_box, device_desc, obeam, oracle_job_xyz, oscene, rel_l1
 
 pytestmark = pytest.mark.gpu
 
@@ -144,3 +144,37 @@ def test_rays_without_a_direction(ctx, direction):
     p = oracle.vol_params(32, 32, 9, max_dist=9.0, max_bounces=5)
     assert num.tolist() == [oracle.simulate_photon(oscene(scene), obeam(beam), p, i)[0] for i in range(64)]
     f.close()
+
+
+def test_films_of_three_bins_are_spectral(ctx):
+    """The images of a film of three bins (film object, allocation-free call, batch,
+    plain launches) are its bins times the bin-averaged colour-matching functions."""
+    import torch
+    n, w, h = 20_000, 64, 48
+    weights = oracle.bin_weights(3, 380.0, 730.0).astype(np.float64)
+    f = _dsotm(ctx, n, w, h, bins=3)
+    f.trace_and_resolve(n, 3)
+    raw = f.read_raw().reshape(-1, 3).astype(np.float64)
+    # three f64 products and sums, rounded to f32 once
+    expect = (raw @ weights.T).reshape(-1) * 2.0 ** -32
+    assert raw.sum() > 0 and np.abs(f.accum() - expect).max() <= 2.0 ** -23 * expect.max()
+    scene, beam, cam = sb.dsotm_scene(w / h)
+    keep = []
+    desc = device_desc(sb, _lib, torch, scene, cam, beam, w, h, 3, 3, keep)
+    xyz = torch.empty(3 * w * h, dtype=torch.float32, device="cuda")
+    _lib.check(_lib.lib.sc_trace_xyz_noalloc(sb.sample_tables().ctypes.data_as(C.POINTER(C.c_float)), C.byref(desc),
+                                             0, n, C.c_void_p(xyz.data_ptr()), None))
+    torch.cuda.synchronize()
+    assert np.array_equal(xyz.cpu().numpy(), f.accum())
+    f.close()
+    job = prism_jobs(specs.random_prism_jobs(1, 3, 3, photons=(20_000, 20_000), side=(40, 60)))
+    j = job[0]
+    b = Batch(ctx, job)
+    images = []
+    for run in (b.run, b.run_plain):
+        run()
+        b.synchronize()
+        images.append(b.read_all_xyz())
+    b.close()
+    ref = oracle_job_xyz(j)
+    assert ref.sum() > 0 and np.array_equal(images[0], images[1]) and rel_l1(images[0], ref) < 2e-3
