@@ -161,6 +161,12 @@ __global__ void __launch_bounds__(256) zbuffer_kernel(sc_camera cam, uint32_t w,
 // The calls' device memory comes from the context's pool, on the default stream that
 // they run on: a cudaMalloc and a cudaFree for each buffer of each call, which also
 // wait for the device, took 1.3 of the 2.3 ms of a 512x512 caustic of 2^18 photons.
+// The pool keeps what it is given back until the context goes, so a call that takes
+// more than this (a caustic of 1.8 M texels, a z-buffer of 16 M pixels) allocates and frees
+// its image buffers instead, as every call did before.
+constexpr size_t kPooledCallBytes = 64u << 20;
+cudaMemPool_t call_pool(const sc_ctx* ctx, size_t bytes) { return bytes <= kPooledCallBytes ? ctx->pool : nullptr; }
+
 int upload_scene(const sc_ctx* ctx, const sc_primitive* prims, uint32_t np, const sc_plane* planes, uint32_t npl,
                  const sc_material* mats, uint32_t nm, DevBuf<sc_primitive>& dp, DevBuf<sc_plane>& dpl,
                  DevBuf<sc_material>& dm) {
@@ -209,7 +215,8 @@ int sc_lighttrace(sc_ctx* ctx, const sc_primitive* prims, uint32_t n_prims, cons
     const size_t n = 3ull * width * height;
     DevBuf<unsigned long long> film;
     DevBuf<float> out;
-    film.bind(ctx->pool, 0); out.bind(ctx->pool, 0);
+    const cudaMemPool_t pool = call_pool(ctx, n * (sizeof(unsigned long long) + sizeof(float)));
+    film.bind(pool, 0); out.bind(pool, 0);
     SC_CUDA(film.alloc(n));
     SC_CUDA(out.alloc(n));
     SC_CUDA(cudaMemsetAsync(film.p, 0, film.bytes(), 0));
@@ -253,7 +260,7 @@ int sc_scene_zbuffer(sc_ctx* ctx, const sc_primitive* prims, uint32_t n_prims, c
     int rc = upload_scene(ctx, prims, n_prims, planes, n_planes, mats, n_mats, dp, dpl, dm);
     if (rc != SC_OK) return rc;
     DevBuf<float> z;
-    z.bind(ctx->pool, 0);
+    z.bind(call_pool(ctx, (size_t)width * height * sizeof(float)), 0);
     SC_CUDA(z.alloc((size_t)width * height));
     const size_t smem = n_prims * sizeof(sc_primitive) + n_planes * sizeof(sc_plane) + n_mats * sizeof(sc_material);
     dim3 block(16, 16), grid((width + 15) / 16, (height + 15) / 16);

@@ -178,3 +178,20 @@ def test_films_of_three_bins_are_spectral(ctx):
     b.close()
     ref = oracle_job_xyz(j)
     assert ref.sum() > 0 and np.array_equal(images[0], images[1]) and rel_l1(images[0], ref) < 2e-3
+
+
+def test_large_calls_give_their_memory_back(ctx):
+    """A caustic and a z-buffer of more memory than a context keeps leave the
+    device's free memory as it was."""
+    import torch
+    scene, beam, cam = sb.dsotm_scene(1.0)
+    screen = sb.Screen((-4.0, -1.0, -4.0), (8.0, 0.0, 0.0), (0.0, 0.0, 8.0), 64, 64)
+    sb.trace(ctx, scene, screen, beam, 1000, 3)  # kernels loaded
+    sb.scene_zbuffer(ctx, scene, cam, 64, 64)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    large = sb.Screen((-4.0, -1.0, -4.0), (8.0, 0.0, 0.0), (0.0, 0.0, 8.0), 4096, 4096)  # 604 MB
+    sb.trace(ctx, scene, large, beam, 1000, 3)
+    sb.scene_zbuffer(ctx, scene, cam, 8192, 4096)  # 134 MB
+    assert large.sum.sum() > 0
+    assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
