@@ -151,11 +151,11 @@ __device__ __forceinline__ uint64_t tent2(uint64_t dx2, uint64_t dy, uint64_t ni
     return pack2(fmaxf(a, 0.0f), fmaxf(b, 0.0f));
 }
 
-// Fixed-point value of an already scaled, non-negative deposit: the same
-// integer as to_fixed(x, scale) for y = x * scale (scale a power of two), with
-// the common case (y < 2^23) in two ALU operations and no sign test.
+// Fixed-point value of an already scaled deposit: the same integer as
+// to_fixed(x, scale) for y = x * scale (scale a power of two), with the common case
+// (0 <= y < 2^23, by its bits) in two ALU operations.
 __device__ __forceinline__ unsigned long long fixed_scaled(float y) {
-    if (y < 8388608.0f) return (unsigned long long)(__float_as_uint(y + 8388608.0f) - 0x4B000000u);
+    if (__float_as_uint(y) < 0x4B000000u) return (unsigned long long)(__float_as_uint(y + 8388608.0f) - 0x4B000000u);
     return to_fixed(y, 1.0f);
 }
 

@@ -195,3 +195,12 @@ def test_large_calls_give_their_memory_back(ctx):
     sb.scene_zbuffer(ctx, scene, cam, 8192, 4096)  # 134 MB
     assert large.sum.sum() > 0
     assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
+
+
+@pytest.mark.parametrize("bins", [0, 16])
+@pytest.mark.parametrize("weights", [(-0.5, 0.06, 0.5), (0.5, 0.06, 1.2)])
+def test_beam_weights_below_zero_leave_a_film_black(ctx, bins, weights):
+    f = _dsotm(ctx, 500, weights=sb.VolWeights(*weights), bins=bins, estimator=sb.BEAM)
+    f.trace_and_resolve(500, 3)
+    assert not f.read_raw().any()
+    f.close()
