@@ -198,6 +198,20 @@ def test_large_calls_give_their_memory_back(ctx):
 
 
 @pytest.mark.parametrize("bins", [0, 16])
+@pytest.mark.parametrize("g", [0.0, 0.4])
+def test_free_flight_samples_with_and_without_a_z_buffer(ctx, bins, g):
+    """A z-buffer that hides nothing has its samples worked out one by one: the
+    same cells as the four of a segment together."""
+    raws = []
+    for z in (None, np.full(64 * 48, np.inf, np.float32)):
+        f = _dsotm(ctx, 50_000, weights=sb.VolWeights(0.5, 0.3, g), bins=bins, estimator=3, zbuffer=z)
+        f.trace_and_resolve(50_000, 3)
+        raws.append(f.read_raw())
+        f.close()
+    assert raws[0].sum() > 0 and np.array_equal(raws[0], raws[1])
+
+
+@pytest.mark.parametrize("bins", [0, 16])
 @pytest.mark.parametrize("weights", [(-0.5, 0.06, 0.5), (0.5, 0.06, 1.2)])
 def test_beam_weights_below_zero_leave_a_film_black(ctx, bins, weights):
     f = _dsotm(ctx, 500, weights=sb.VolWeights(*weights), bins=bins, estimator=sb.BEAM)
