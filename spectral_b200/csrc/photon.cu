@@ -33,12 +33,14 @@ __host__ __device__ __forceinline__ size_t park_offset(const PhotonParams& p, ui
     return (b + 15u) & ~size_t(15);
 }
 
-// 256 threads per CTA; MINB CTAs per SM bound the registers (4: 63 registers,
-// no spills; 5: 48 registers, a few spills, more warps in flight).
+// 256 threads per CTA; MINB CTAs per SM bound the registers (4: 64 registers, spectral
+// films without spills, XYZ films with 24 B, with the cache 38 B; 5: 48 registers, 140 B
+// and 240 to 300 B, more warps in flight).
 // FF: built with free-flight sampling (estimator 3) as well.  EXACT: haze
 // samples in the CPU crate's operation order.  CACHE: built with the shared-memory
 // cell cache.  chunk: photons of each warp.  cached: slots of
-// the cache, 0: none (CACHE only).
+// the cache, 0: none (CACHE only; launches without it take the kernel without it: XYZ,
+// dsotm 640x360, 2^14 photons 32.8 -> 30.3 us, rainbow 25.9 -> 24.0).
 template <bool SPEC, int AGG, int MINB, bool FF, bool EXACT = false, bool CACHE = false>
 __global__ void __launch_bounds__(256, MINB) photon_kernel(const PhotonParams p, uint32_t mask_words, uint32_t chunk,
                                                            uint32_t cached) {
@@ -276,32 +278,23 @@ size_t scene_smem_bytes(uint32_t n_prims, uint32_t n_planes, uint32_t n_mats) {
 
 using PhotonKernelFn = void (*)(const PhotonParams, uint32_t, uint32_t, uint32_t);
 
-// `few`: film of few cells per pixel (the kernels built with the cell cache).
-static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool few, bool ff, bool exact = false) {
-    // haze samples in the reference's operation order: plain atomics, 4 CTAs per SM
+// `cached`: the launch takes the cell cache (the kernels built with it).
+template <bool SPEC>
+static PhotonKernelFn photon_fn(const LaunchShape& s, bool cached, bool ff, bool exact) {
+    // haze samples in the reference's operation order, and free-flight launches: plain
+    // atomics, 4 CTAs per SM
     if (exact) {
-        if (ff) {
-            if (!spec) return photon_kernel<false, 0, 4, true, true, true>;
-            return few ? photon_kernel<true, 0, 4, true, true, true> : photon_kernel<true, 0, 4, true, true>;
-        }
-        if (!spec) return photon_kernel<false, 0, 4, false, true, true>;
-        return few ? photon_kernel<true, 0, 4, false, true, true> : photon_kernel<true, 0, 4, false, true>;
+        if (ff) return cached ? photon_kernel<SPEC, 0, 4, true, true, true> : photon_kernel<SPEC, 0, 4, true, true>;
+        return cached ? photon_kernel<SPEC, 0, 4, false, true, true> : photon_kernel<SPEC, 0, 4, false, true>;
     }
-    // free-flight launches: plain atomics, 4 CTAs per SM
-    if (ff) {
-        if (!spec) return photon_kernel<false, 0, 4, true, false, true>;
-        return few ? photon_kernel<true, 0, 4, true, false, true> : photon_kernel<true, 0, 4, true>;
-    }
-    if (s.aggregate) {
-        if (s.minb >= 5) return spec ? photon_kernel<true, 1, 5, false> : photon_kernel<false, 1, 5, false>;
-        return spec ? photon_kernel<true, 1, 4, false> : photon_kernel<false, 1, 4, false>;
-    }
-    if (few) {  // with the cache, 4 or 3 CTAs per SM (cache_slots)
-        return spec ? photon_kernel<true, 0, 4, false, false, true> : photon_kernel<false, 0, 4, false, false, true>;
-    }
-    return s.minb >= 5 ? photon_kernel<true, 0, 5, false> : photon_kernel<true, 0, 4, false>;
+    if (ff) return cached ? photon_kernel<SPEC, 0, 4, true, false, true> : photon_kernel<SPEC, 0, 4, true>;
+    if (s.aggregate) return s.minb >= 5 ? photon_kernel<SPEC, 1, 5, false> : photon_kernel<SPEC, 1, 4, false>;
+    if (cached) return photon_kernel<SPEC, 0, 4, false, false, true>;  // 4 or 3 CTAs per SM (cache_slots)
+    return s.minb >= 5 ? photon_kernel<SPEC, 0, 5, false> : photon_kernel<SPEC, 0, 4, false>;
 }
-static bool few_cells(bool spec, uint32_t channels) { return !spec || channels <= kCacheBins; }
+static PhotonKernelFn photon_fn(const LaunchShape& s, bool spec, bool cached, bool ff, bool exact = false) {
+    return spec ? photon_fn<true>(s, cached, ff, exact) : photon_fn<false>(s, cached, ff, exact);
+}
 // Shared memory beyond scene + mask: the parked photons of 8 warps.
 static size_t park_bytes(bool spec) {
     return 16 + 8 * (spec ? sizeof(ParkedPhotons<true>) : sizeof(ParkedPhotons<false>));
@@ -360,7 +353,7 @@ int occupancy_blocks(const void* fn, int block, size_t smem) {
 }
 
 int photon_occupancy_blocks(const LaunchShape& shape, bool spectral, size_t smem) {
-    return occupancy_blocks(reinterpret_cast<const void*>(photon_fn(shape, spectral, !spectral, false)),
+    return occupancy_blocks(reinterpret_cast<const void*>(photon_fn(shape, spectral, false, false)),
                             (int)shape.block, smem + park_bytes(spectral));
 }
 
@@ -498,7 +491,7 @@ static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& 
     set_haze_consts(p);
     const bool exact = p.haze_exact != 0u;
     const uint32_t mw = photon_mask_words(p);
-    const bool spec = p.channels != 3u || p.bins != 0u, few = few_cells(spec, p.channels);
+    const bool spec = p.channels != 3u || p.bins != 0u, few = !spec || p.channels <= kCacheBins;  // cells per pixel
     // 32 photons for each warp while the GPU holds all of them; then about two
     // chunks for each warp that it holds, 64 to 256 photons: the hardware starts
     // the next CTA where one has ended.  One CTA per resident slot with its share
@@ -515,7 +508,7 @@ static cudaError_t launch_photons_in(const PhotonParams& p0, const LaunchShape& 
     size_t smem = park_offset(p, mw) + park_bytes(spec);
     const uint32_t slots = cached ? cache_slots(spec, smem, chunk, pixels) : 0u;
     smem += slots * (size_t)(spec ? CellCacheOf<true>::kSlotBytes : CellCacheOf<false>::kSlotBytes);
-    const PhotonKernelFn fn = photon_fn(shape, spec, few, free_flight(p), exact);
+    const PhotonKernelFn fn = photon_fn(shape, spec, slots != 0u, free_flight(p), exact);
     if (smem > 48 * 1024) allow_max_smem(reinterpret_cast<const void*>(fn));
     // a launch of less than one and a half rounds of CTAs is spread over one (dsotm
     // 400x300, 2^18 photons: 107 -> 90 us); with more rounds, chunks that are no multiple
