@@ -453,8 +453,14 @@ cudaError_t launch_photons(const PhotonParams& p, const LaunchShape& shape, cuda
 // 933 -> 385, 2^22 3243 -> 1300; dsotm 800x800, 4M photons 1161 -> 800; 8 bins, 2^20
 // 265 -> 216 (16 bins take 175 without it).  The rainbow's beam (205 pixels): XYZ 2^20
 // 330 -> 278 us (0.055 samples a cell), 2 bins 188 -> 163 (0.028), but 4 bins 108 -> 146
-// and XYZ 2^15 24 -> 29 (0.014): the line lies at 0.02.  A z-buffer takes samples
-// away: 0.055 then lose (148 -> 201), 4 still win (prism 995 -> 464).
+// (0.014): the line lies at 0.02.  At 0.05 for launches of less than 2^16 photons, whose
+// one CTA an SM does not hide the clearing and flushing (XYZ, 2^15 photons, rainbow
+// 256x256 (0.027) 26.5 and 30.9 us, 160x160 (0.07) 32.3 and 30.2, 128x128 (0.11) 36.3
+// and 30.1), and for photons of one segment, whose samples no surface gathers (rainbow
+// XYZ, 2^18 (0.028) 38.2 and 40.3, 2^20 (0.055) 124 and 116).  A z-buffer takes samples
+// away: 0.055 then lose (148 -> 201), 4 still win (prism 995 -> 464); and without a scene
+// they spread over all of the beam (XYZ, 95 pixels wide, 2^20 (0.1) 65 and 81, 2^21
+// (0.2) 129 and 139): 0.4.
 static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t chunk, float pixels) {
     if (p.photon_count < (1u << 15)) return false;
     // keys are 32-bit cell indices below CellCache::kFree; films of one to seven rows
@@ -464,7 +470,9 @@ static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t
     // 8 warps of at most 256 photons, 4 samples a segment
     if (8ull * 256ull * 4ull * p.max_bounces > kCacheDeposits) return false;
     if (!(pixels > 0.0f)) return false;
-    return 32.0f * (float)chunk >= (p.zbuf ? 0.4f : 0.02f) * pixels * (float)cells_per_pixel;
+    const float line = p.zbuf || p.n_prims == 0u ? 0.4f
+                       : p.photon_count < (1u << 16) || p.max_bounces == 1u ? 0.05f : 0.02f;
+    return 32.0f * (float)chunk >= line * pixels * (float)cells_per_pixel;
 }
 // Slots of the cell cache beside `smem` bytes of a CTA (228 KB per SM, 1 KB of each
 // CTA taken): what lets 4 CTAs share an SM, or for XYZ films 3, where the hot cells
