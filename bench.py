@@ -68,11 +68,11 @@ METRIC_BEAM = "photons/s (forward + photon-beam estimator, volumetric single sca
 # ncu capture of the default workload on a B200 (the profile summaries give the
 # commands); reported only when the workload runs at its default size.
 NCU_TRAFFIC = {
-    "prism": (2092544, "photon_kernel, one capture"),
-    "rainbow": (4839725056, "order_count + order_scan + order_scatter + photon_kernel, one capture"),
-    "beam": (3842560, "beam_kernel, one capture"),
-    "tracer": (6145474816, "all tracer wave kernels of one accumulate(64), one capture"),
-    "batch": (3953000000, "batch_kernel + reduce_scan + reduce_list, scaled from a capture of the first 64 "
+    "prism": (5587584, "photon_kernel, two launches in one capture"),
+    "rainbow": (1449891584, "order_count + order_scan + order_scatter + photon_kernel, one capture"),
+    "beam": (6201600, "beam_kernel, one capture"),
+    "tracer": (5685271552, "all tracer wave kernels of one accumulate(64), one capture"),
+    "batch": (4336000000, "batch_kernel + reduce_scan + reduce_list, scaled from a capture of the first 64 "
                           "scenes (4.4 GB of films): batch_kernel by photons, reduce_scan by film bytes, reduce_list by "
                           "lit-tile bytes"),
     "atomics": (24887296, "synthetic_splat_kernel, one capture"),
@@ -85,11 +85,11 @@ NCU_TRAFFIC = {
 # active per instruction: the instruction-issue roofline of kernels whose films
 # stay in L2.
 NCU_INST = {
-    "batch": (9731331222 / 2 / 48957886, 26.57, "batch_kernel<0, 4, 0>: two launches on the first 64 scenes "
+    "batch": (9763022737 / 2 / 48957886, 26.57, "batch_kernel<0, 4, 0>: two launches on the first 64 scenes "
                                                  "(48,957,886 photons each), per photon"),
-    "prism": (274675052 / 2 / (1 << 20), 24.67, "photon_kernel: two launches of 2^20 photons, per photon"),
-    "rainbow": (4785072070 / (1 << 26), 23.91, "photon_kernel: one launch of 2^26 photons, per photon"),
-    "tracer": (2577983977 / 58982400, 25.44, "tr_shade, tr_tail, tr_accumulate: the 59 launches of one "
+    "prism": (275535741 / 2 / (1 << 20), 24.67, "photon_kernel: two launches of 2^20 photons, per photon"),
+    "rainbow": (4789949565 / (1 << 26), 23.92, "photon_kernel: one launch of 2^26 photons, per photon"),
+    "tracer": (2578202959 / 58982400, 25.44, "tr_shade, tr_tail, tr_accumulate: the 59 launches of one "
                                              "accumulate(64), per path sample"),
 }
 
@@ -559,10 +559,13 @@ def run_gpu(args, rank, world, local_rank):
         alg_note = "8 B per film channel per in-frame haze sample: %d samples per launch" % splats
         flops = photons * 20 + segments * 14 * npl + segments * 4 * 60 + scatters * 45
     lit_bytes = dirty_tiles * 64 * CH * 8
-    # the library traces photons in film-bin order when a spectral film is larger than L2
-    film_bytes = ((W + 7) // 8) * ((H + 7) // 8) * 64 * CH * 8
-    ordered = (EST != 2 and B > 0 and N >= (1 << 16) and os.environ.get("SPECTRAL_CUDA_ORDER", "1") != "0"
-               and film_bytes > torch.cuda.get_device_properties(dev).L2_cache_size)
+    # the library traces photons in film-bin order where a launch touches more of a spectral
+    # film than L2 holds: the rainbow's wide beam (342 MB of bins under it) from two L2s of
+    # sectors on; the prism's has 0.5 MB
+    order = os.environ.get("SPECTRAL_CUDA_ORDER", "1")
+    l2 = torch.cuda.get_device_properties(dev).L2_cache_size
+    ordered = (EST != 2 and B > 0 and N >= (1 << 16)
+               and (order == "2" or (order == "1" and args.workload == "rainbow" and N * 320 >= 2 * l2)))
     traffic, traffic_src = ncu_traffic(args.workload, not args.photons)
     workload_txt = {"prism": "SF11 prism apex 60 side 1, beam 0.02 @45deg, 2^20 photons, 640x360x64 bins",
                     "rainbow": "water sphere r=1, beam 2.2, 2^26 photons, 1920x1080x64 bins",

@@ -244,7 +244,7 @@ struct sc_batch {
             p.mats = reinterpret_cast<const sc_material*>(
                 reinterpret_cast<const unsigned char*>(d_jobs.p + j) + offsetof(BatchSlotImage, mats));
             // launch order: on these scenes' films it beats the single-film
-            // default (the wavelength-ordered dispatch for films larger than L2)
+            // default (the wavelength-ordered dispatch where a launch touches more than L2 holds)
             LaunchShape shape;
             shape.block = 256; shape.aggregate = 0; shape.minb = 4;
             const size_t smem = scene_smem_bytes(p.n_prims, p.n_planes, p.n_mats) +

@@ -23,8 +23,9 @@
 // through a window of pixels that the lanes hold in registers (window_march).
 // Film width and height are below 2^16 (corners are packed into one word).
 //
-// Bound: instruction issue (0.60 of the issue slots at 24 warps per SM, which
-// registers limit; 4 CTAs per SM spill and are 4-8 % slower on most films).  Of
+// Bound: instruction issue (0.71 of the issue slots at 24 warps per SM, which
+// registers limit: 80, with 202 B of spills; 4 CTAs per SM spill more and are 4-8 %
+// slower on most films).  Of
 // the 38 ms that 2^18 photons take on the 800x800 XYZ film, the setup of the
 // 470 M steps is 13 ms and the windows are the rest, ~75 warp instructions for
 // each of the 279 M steps in frame.  Splatting step by step over each box, with

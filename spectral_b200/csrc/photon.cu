@@ -1,6 +1,6 @@
 // Forward photon emitter / tracer with point-estimator haze splatting.
 //
-// One thread per photon, restating render_volumetric_scene_point
+// One photon per lane, in groups (photon_trace.cuh), restating render_volumetric_scene_point
 // (spectral-core/src/volume.rs:99-168) and its GPU mirror
 // (spectral-gpu/src/shaders/volume.wgsl:542-647): emission from the beam
 // aperture, hero wavelength, up to max_bounces segments, 4 uniform haze samples
@@ -477,9 +477,12 @@ static bool cache_pays(const PhotonParams& p, uint32_t cells_per_pixel, uint32_t
 // Slots of the cell cache beside `smem` bytes of a CTA (228 KB per SM, 1 KB of each
 // CTA taken): what lets 4 CTAs share an SM, or for XYZ films 3, where the hot cells
 // (about 2.5 for each pixel of the beam) find a slot then but not among 4 CTAs, and
-// where chunks are long, or the beam is very wide, and they do neither way.  4 against 3 CTAs, 2^20 photons: 1 to 8
-// bins 217 and 249 us, dsotm XYZ 256x256 205 and 242, 800x800 239 and 281; prism 640x360
-// XYZ 415 and 384 (2^22: 1388 and 1296), dsotm 1600x1200 2^22 955 and 900.  Launches of
+// where chunks are long, or the beam is very wide, and they do neither way.  4 against 3
+// CTAs, 2^20 photons: 1 to 8 bins 217 and 249 us, dsotm XYZ 256x256 205 and 242, 800x800
+// 239 and 281; prism 640x360 XYZ 415 and 384 (2^22: 1388 and 1296), dsotm 1600x1200 2^22
+// 955 and 900.  Very wide (rainbow XYZ 640x360, hot 100 n): 2^18 88 and 85 us, 2^19 155
+// and 144, 2^20 282 and 254, 2^21 535 and 464 (256x256, 50 n: 2^17 55 and 57, 2^18 88 and
+// 85, 2^20 277 and 250); no beam between 8 and 50 n was measured.  Launches of
 // 32 photons a warp clear and flush 2048 at most (2^16 photons: 42 us against 44).
 static uint32_t cache_slots(bool spec, size_t smem, uint32_t chunk, float pixels) {
     const size_t slot = spec ? CellCacheOf<true>::kSlotBytes : CellCacheOf<false>::kSlotBytes;

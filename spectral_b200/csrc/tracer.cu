@@ -340,7 +340,8 @@ __global__ void __launch_bounds__(kShadeThreads, kStageCtasPerSm) tr_shade(const
 // at entry), whatever bounces the others are at.  Warps
 // stay full without waiting for one another.  The same hit and shade code, so the
 // image is unchanged.  Segments after each path's first tail bounce are added to
-// counts[first + 1].
+// counts[first + 1].  (16, 20, 24, 28, 32 lanes: accumulate(64) with its read-back 3.83,
+// 3.82 to 3.87, 3.76 to 3.80, 3.80, 3.85 to 3.91 ms.)
 constexpr uint32_t kTailLive = 24;
 __global__ void __launch_bounds__(256, kStageCtasPerSm) tr_tail(const TracerParams* __restrict__ gp, uint32_t first,
                                                                 RayQueue q, uint32_t* counts, float* result) {
@@ -460,7 +461,11 @@ cudaError_t launch_tracer_wave(const TracerParams* d_params, const TracerLaunch&
     // the first bounce makes, intersects and shades the primary rays in one kernel
     // (where the caller does not say: two, or one for waves that the tail's warps
     // hold with few refills.  accumulate(64) at 1280x720, waves of 2^22 paths: one 3.28
-    // ms, two 3.05, three 3.06; accumulate(4) at 333x187: 54, 60, 64 us)
+    // ms, two 3.05, three 3.06; accumulate(4) at 333x187: 54, 60, 64 us.  One and two by
+    // the wave's paths: the prism on its floor under a black sky 2^18 54 and 60 us, 2^19
+    // 75 and 72, 2^20 102 and 98, 2^21 178 and 171, 2^22 285 and 274, under a bright one
+    // 2^20 106 and 108, 2^21 197 and 188; glass under a sky, whose paths end after fewer
+    // bounces, 2^20 92 and 98, 2^22 239 and 251)
     const uint32_t want = L.wave_bounces ? L.wave_bounces : n_paths <= (1u << 20) ? 1u : 2u;
     const uint32_t wave_bounces = L.max_depth < want ? L.max_depth : want;
     // bounce b intersects and shades the rays of bounce b and queues its
