@@ -750,8 +750,16 @@ def run_gpu_tracer(args, rank, world, local_rank):
     # XYZ (12 B) written and read by the per-pixel sums
     qbytes = (segments - samples) * 2 * 44 + samples * 2 * 12
     wave_paths = 1 << args.tracer_wave_log2 if args.tracer_wave_log2 else TRACER_WAVE_PATHS
+    per_wave = max(1, wave_paths // SPP)  # pixels
+
+    def wave_launches(pixels):
+        # compacted bounces (the first makes the primary rays; by default two, one in waves
+        # of up to 2^20 paths), the tail, per-pixel sums
+        b = min(kw["max_depth"], args.tracer_wave_bounces or (1 if pixels * SPP <= 1 << 20 else 2))
+        return b + (1 if kw["max_depth"] > b else 0) + 1
+
+    launches = sum(wave_launches(min(per_wave, W * H - at)) for at in range(0, W * H, per_wave))
     wb = args.tracer_wave_bounces or 2
-    waves = -(-(W * H) // max(1, wave_paths // SPP))
     line = {
         "metric": "path samples/s (hero-wavelength camera tracer, 4 lanes, depth 8)",
         "value": value, "unit": "samples/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -765,9 +773,7 @@ def run_gpu_tracer(args, rank, world, local_rank):
         "e2e": {"value": e2e_value, "unit": "samples/s", "h2d_bytes_per_step": C.sizeof(cam.c),
                 "d2h_bytes_per_step": 3 * W * H * 4,
                 "path": "sc_tracer_set_camera + clear_accum + accumulate(64) + read_xyz (host f32 XYZ)"},
-        # per wave: two shades (the first makes and intersects the primary rays
-        # and intersects the second bounce's rays), the tail, per-pixel sums
-        "gpu_launches": args.steps * waves * (min(kw["max_depth"], wb) + (1 if kw["max_depth"] > wb else 0) + 1),
+        "gpu_launches": args.steps * launches,
         "kernels": {"accumulate_ms": statistics.mean(step_ms)},
         "roofline": {"bound": "hbm", "achieved": qbytes / step_s / 1e9, "peak": hbm, "unit": "GB/s",
                      "frac": qbytes / step_s / 1e9 / hbm, "traffic": ncu_traffic("tracer")[0],
