@@ -11,7 +11,7 @@ import pytest
 
 import oracle
 import spectral_b200 as sb
-from spectral_b200 import _lib, specs
+from spectral_b200 import _lib, scenes, specs
 from spectral_b200.batch import Batch, prism_jobs
 from helpers import axis_box, device_desc, obeam, oracle_job_xyz, oscene, rel_l1
 
@@ -217,4 +217,25 @@ def test_beam_weights_below_zero_leave_a_film_black(ctx, bins, weights):
     f = _dsotm(ctx, 500, weights=sb.VolWeights(*weights), bins=bins, estimator=sb.BEAM)
     f.trace_and_resolve(500, 3)
     assert not f.read_raw().any()
+    f.close()
+
+
+# samples a cell (32 x photons a warp / pixels under the beam) on both sides of the lines:
+# empty scenes 0.4, single segments and launches below 2^16 photons 0.05, others 0.02
+@pytest.mark.parametrize("name,w,h,n,kw", [
+    ("prism", 96, 64, 40_000, {}), ("rainbow", 96, 64, 40_000, {}),
+    ("rainbow", 200, 200, 65_535, {}), ("rainbow", 200, 200, 65_536, {}),
+    ("rainbow", 128, 128, 65_535, dict(max_bounces=1)), ("rainbow", 256, 256, 65_536, dict(max_bounces=1))])
+@pytest.mark.parametrize("empty", [False, True])
+def test_cell_cache_on_both_sides_of_its_lines(ctx, name, w, h, n, kw, empty):
+    d = {"prism": specs.prism_scene, "rainbow": specs.rainbow_scene}[name]()
+    scene = sb.Scene(background=0.0) if empty else scenes.scene_from_spec(d)
+    f = sb.GpuPhotonFilm(ctx, scene, sb.Camera.look_at(*d["camera"], w / h), sb.Beam(*d["beam"]), w, h, n, 5, 8.0,
+                         sb.VolWeights(0.3, 0.05, 0.0), **kw)
+    f.trace_and_resolve(n, 5)
+    whole = f.read_raw()
+    f.clear_film()
+    for a in range(0, n, 30_011):  # too small for the cache
+        f.dispatch_photons(a, min(a + 30_011, n), 5)
+    assert whole.sum() > 0 and np.array_equal(f.read_raw(), whole)
     f.close()
