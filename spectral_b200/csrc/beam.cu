@@ -643,7 +643,9 @@ cudaError_t launch_beam(const PhotonParams& p, const LaunchShape& shape, cudaStr
     const bool spec = p.channels != 3u || p.bins != 0u;
     const uint32_t need = (p.photon_count - 1u) / 8u + 1u;  // at least one photon per warp
     const uint32_t grid = need < shape.grid ? need : shape.grid;
-    beam_fn(spec)<<<grid, 256, beam_smem(p, mw), s>>>(p, mw);
+    const size_t smem = beam_smem(p, mw);  // the scene may have grown since the film was created
+    if (smem > 48 * 1024) allow_max_smem(reinterpret_cast<const void*>(beam_fn(spec)));
+    beam_fn(spec)<<<grid, 256, smem, s>>>(p, mw);
     return cudaGetLastError();
 }
 

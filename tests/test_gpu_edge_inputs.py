@@ -5,6 +5,9 @@ context keeps.
 
 Films are sums of exact integers: every cell is compared."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -14,6 +17,8 @@ import spectral_b200 as sb
 from spectral_b200 import _lib, scenes, specs
 from spectral_b200.batch import Batch, prism_jobs
 from helpers import axis_box, device_desc, obeam, oracle_job_xyz, oscene, rel_l1
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 pytestmark = pytest.mark.gpu
 
@@ -239,3 +244,25 @@ def test_cell_cache_on_both_sides_of_its_lines(ctx, name, w, h, n, kw, empty):
         f.dispatch_photons(a, min(a + 30_011, n), 5)
     assert whole.sum() > 0 and np.array_equal(f.read_raw(), whole)
     f.close()
+
+
+def test_beam_film_whose_scene_grows():
+    """A beam film created for a small scene takes the largest one afterwards.  In a
+    process of its own: no other film has raised the kernel's shared memory there."""
+    code = """
+import spectral_b200 as sb
+ctx = sb.GpuContext(0)
+scene, beam, cam = sb.dsotm_scene(1.0)
+f = sb.GpuPhotonFilm(ctx, scene, cam, beam, 320, 320, 200, 3, 14.0, sb.VolWeights(), estimator=sb.BEAM)
+f.trace_and_resolve(200, 3)
+one = f.read_raw()
+box = [((1, 0, 0), -1e3), ((-1, 0, 0), -1e3), ((0, 1, 0), -1e3), ((0, -1, 0), -1e3)]
+for i in range(50):  # far behind every photon and the camera
+    scene.add_solid([((0, 0, 1), 1e3 + i), ((0, 0, -1), -1e3 - i - 0.5)] + box[:3], sb.Lambertian(0.5))
+f.set_scene(scene, cam, beam)
+f.clear_film()
+f.trace_and_resolve(200, 3)
+assert one.sum() > 0 and (f.read_raw() == one).all()
+"""
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
