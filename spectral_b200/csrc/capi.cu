@@ -592,10 +592,17 @@ int sc_photon_film_read_raw(sc_photon_film* f, int64_t* out) {
     SC_CUDA(cudaMemcpyAsync(tiles.data(), f->film.p, f->film.bytes(), cudaMemcpyDeviceToHost, f->stream));
     SC_CUDA(cudaStreamSynchronize(f->stream));
     const FilmGeom& g = f->geom;
-    for (uint32_t py = 0; py < g.h; ++py)
-        for (uint32_t px = 0; px < g.w; ++px)
-            for (uint32_t c = 0; c < g.channels; ++c)
-                out[((size_t)py * g.w + px) * g.channels + c] = tiles[film_cell(px, py, g.tiles_x, g.channels, c)];
+    // tile by tile: a tile's cells lie together, bin by bin
+    for (uint32_t y0 = 0; y0 < g.h; y0 += 8u)
+        for (uint32_t x0 = 0; x0 < g.w; x0 += 8u) {
+            const int64_t* tile = tiles.data() + (size_t)film_tile(x0, y0, g.tiles_x) * kTilePixels * g.channels;
+            for (uint32_t py = y0; py < std::min(y0 + 8u, g.h); ++py)
+                for (uint32_t px = x0; px < std::min(x0 + 8u, g.w); ++px) {
+                    const int64_t* cell = tile + film_local(px, py);
+                    int64_t* o = out + ((size_t)py * g.w + px) * g.channels;
+                    for (uint32_t c = 0; c < g.channels; ++c) o[c] = cell[(size_t)c * kTilePixels];
+                }
+        }
     return SC_OK;
     SC_GUARD_END
 }
