@@ -236,13 +236,17 @@ int sc_ctx_create(int device, const float* tables, sc_ctx** out) {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
-    if (cudaMemPoolCreate(&c->pool, &props) == cudaSuccess) {
-        uint64_t keep = UINT64_MAX;
-        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    } else {
-        cudaGetLastError();
-        c->pool = nullptr;  // no pool: photon launches run in launch order
-    }
+    auto make_pool = [&](uint64_t keep) {
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return cudaMemPool_t(nullptr);
+        }
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        return pool;
+    };
+    c->pool = make_pool(UINT64_MAX);  // without it photon launches run in launch order
+    c->call_pool = make_pool(kPooledCallBytes);
     *out = c;
     return SC_OK;
     SC_GUARD_END
@@ -255,10 +259,9 @@ int sc_ctx_destroy(sc_ctx* ctx) {
         DeviceGuard g(ctx->device);
         ctx->cmf.reset();
         ctx->binw_cache.clear();
-        if (ctx->pool) {
-            cudaDeviceSynchronize();  // frees still queued on streams return their blocks first
-            cudaMemPoolDestroy(ctx->pool);
-        }
+        if (ctx->pool || ctx->call_pool) cudaDeviceSynchronize();  // frees still queued on streams return their blocks first
+        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+        if (ctx->call_pool) cudaMemPoolDestroy(ctx->call_pool);
     }
     delete ctx;
     return SC_OK;

@@ -94,6 +94,8 @@ struct DevBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
+constexpr uint64_t kPooledCallBytes = 64u << 20;
+
 }  // namespace sc
 
 struct sc_ctx {
@@ -105,6 +107,10 @@ struct sc_ctx {
     // stream-ordered scratch (the wavelength-ordered photon dispatch); memory
     // freed to it stays reserved for the next launch until the context goes
     cudaMemPool_t pool = nullptr;
+    // scratch of the caustic and z-buffer calls, which run on the default stream: a pool of
+    // their own, since a film that took memory from it would wait for that stream (a film
+    // created after a caustic 175 -> 201 us); keeps sc::kPooledCallBytes at most
+    cudaMemPool_t call_pool = nullptr;
     std::mutex mu;
     // bin-averaged CMF weights of spectral films reduced through the
     // device-pointer API, per (bins, band); freed with the context

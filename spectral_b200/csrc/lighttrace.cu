@@ -158,21 +158,20 @@ __global__ void __launch_bounds__(256) zbuffer_kernel(sc_camera cam, uint32_t w,
     out[(size_t)py * w + px] = t_scene < t_floor ? t_scene : t_floor;
 }
 
-// The calls' device memory comes from the context's pool, on the default stream that
+// The calls' device memory comes from a pool of the context's, on the default stream that
 // they run on: a cudaMalloc and a cudaFree for each buffer of each call, which also
 // wait for the device, took 1.3 of the 2.3 ms of a 512x512 caustic of 2^18 photons.
-// The pool keeps what it is given back until the context goes, so a call that takes
-// more than this (a caustic of 1.8 M texels, a z-buffer of 16 M pixels) allocates and frees
-// its image buffers instead, as every call did before.
-constexpr size_t kPooledCallBytes = 64u << 20;
-cudaMemPool_t call_pool(const sc_ctx* ctx, size_t bytes) { return bytes <= kPooledCallBytes ? ctx->pool : nullptr; }
+// The pool keeps kPooledCallBytes, so a call that takes more (a caustic of 1.8 M texels, a
+// z-buffer of 16 M pixels) allocates and frees its image buffers instead, as every call did
+// before.
+cudaMemPool_t call_pool(const sc_ctx* ctx, size_t bytes) { return bytes <= kPooledCallBytes ? ctx->call_pool : nullptr; }
 
 int upload_scene(const sc_ctx* ctx, const sc_primitive* prims, uint32_t np, const sc_plane* planes, uint32_t npl,
                  const sc_material* mats, uint32_t nm, DevBuf<sc_primitive>& dp, DevBuf<sc_plane>& dpl,
                  DevBuf<sc_material>& dm) {
     const int rc = check_scene(np, npl, nm, prims, planes, mats);
     if (rc != SC_OK) return rc;
-    dp.bind(ctx->pool, 0); dpl.bind(ctx->pool, 0); dm.bind(ctx->pool, 0);
+    dp.bind(ctx->call_pool, 0); dpl.bind(ctx->call_pool, 0); dm.bind(ctx->call_pool, 0);
     SC_CUDA(dp.alloc(np ? np : 1));
     SC_CUDA(dpl.alloc(npl ? npl : 1));
     SC_CUDA(dm.alloc(nm ? nm : 1));
